@@ -22,6 +22,7 @@
 #include "bucket_sum.cuh"
 #include "device_util.cuh"
 #include "kernels.h"
+#include "tensor_mul.cuh"
 
 #include <algorithm>
 #include <cstring>
@@ -580,6 +581,8 @@ struct FlatArgs {
     Fp *tot, *totinv;    // per warp: product of all, and its inverse
     size_t slots;
     int n_lists;
+    uint32_t *err; // error words, marked when a wait for the tensor core gives up (may be null)
+    uint32_t n_err;
 };
 
 // Entry idx of the digit table (kCombEntryBytes apart).
@@ -597,24 +600,103 @@ __device__ __forceinline__ size_t comb_index(const FlatArgs &a, uint32_t o, uint
     return (size_t)(o % kCells) * a.per_j + (size_t)i * a.per_i + a.win.entry_off((int)k) + (uint32_t)(abs(v) - 1);
 }
 
+// The products of the round kernels below run on the tensor cores
+// (tensor_mul.cuh), a group of kTmGroup lanes at a time: every lane of a group
+// walks as many pairs as the group's longest share, its own spare ones neutral
+// (denominator one, nothing stored).  Shares differ by one pair at most, and
+// lanes of lower index have the longer ones.
+__device__ __forceinline__ int group_steps(uint32_t P, uint32_t gl, uint32_t NL) {
+    const uint32_t first = gl & ~(uint32_t)(kTmGroup - 1);
+    return P > first ? (int)((P - first + NL - 1) / NL) : 0;
+}
+
 // End of every pass-1 kernel: the product of the other lanes' running products
 // for each lane, and the warp's product of all of them.  A butterfly over the
 // lanes: at level k each lane multiplies in the product of the partner group
 // of 2^k lanes (lane ^ 2^k's group), so after five levels every lane holds the
 // total, and the five partner groups' products together are the other lanes':
 // 9 products per lane, against 11 for a prefix and a suffix scan.
-__device__ __forceinline__ void flat_pass1_products(const Fp &acc, Fp *others, Fp *tot, size_t gl, size_t wg) {
+template <class G>
+__device__ __forceinline__ void flat_pass1_products(G &g, const Fp &acc, Fp *others, Fp *tot, size_t gl, size_t wg) {
     const int lane = threadIdx.x & 31;
     Fp group = acc, rest = fp_shfl_xor(acc, 1);
-    group = fp_mul(group, rest);
+    group = tm_mul<false>(g, group, rest);
 #pragma unroll 1
     for (int d = 2; d < 32; d <<= 1) {
         const Fp partner = fp_shfl_xor(group, d);
-        rest = fp_mul(rest, partner);
-        group = fp_mul(group, partner);
+        rest = tm_mul<false>(g, rest, partner);
+        group = tm_mul<true>(g, group, partner);
     }
     st_vec(&others[gl], rest);
     if (lane == 0) st_vec(&tot[wg], group);
+}
+
+// An affine point in memory, its sign flipped when neg; null: infinity.
+struct PointRef {
+    const G1A *p;
+    bool neg;
+    __device__ __forceinline__ Fp x() const { return p ? ld_vec(&p->x) : fp_zero(); }
+    __device__ __forceinline__ Fp y() const {
+        if (!p) return fp_zero();
+        const Fp v = ld_vec(&p->y);
+        return neg ? fp_neg(v) : v;
+    }
+    __device__ __forceinline__ G1A point() const { return G1A{x(), y()}; }
+};
+
+// Pass 1 of one pair: its denominator into the lane's running product, the
+// product so far to the prefix slot.
+template <class G, class A, class B>
+__device__ __forceinline__ void pass1_pair(G &g, Fp &acc, bool active, uint32_t *pre, int s, A a, B b) {
+    Fp den = fp_one();
+    if (active) {
+        wb_store_pre(pre, s, acc);
+        den = pair_denominator_x(a.x(), b.x(), [&] { return a.point(); }, [&] { return b.point(); });
+    }
+    acc = tm_mul<false>(g, acc, den);
+}
+
+// Pass 2 of one pair: its inverse denominator out of the running inverse, and the
+// sum to out.  The points are read again where they are needed (they are in
+// shared memory or in L1 by then) instead of being held across the products.
+template <class G, class A, class B>
+__device__ __forceinline__ void pass2_pair(G &g, Fp &inv, bool active, const uint32_t *pre, int t, A a, B b,
+                                           G1A *out) {
+    Fp den = fp_one(), num = fp_one(), lam = fp_one();
+    int kind = 0;
+    if (active) {
+        lam = wb_load_pre(pre, t);
+        const G1A p = a.point(), q = b.point();
+        kind = pair_kind(p, q);
+        den = pair_denominator(p, q, kind);
+        if (kind == 1) {
+            const Fp xx = fp_sqr(p.x);
+            num = fp_add(fp_dbl(xx), xx);
+        } else {
+            num = fp_sub(q.y, p.y);
+        }
+    }
+    lam = tm_mul<false>(g, inv, lam);
+    inv = tm_mul<false>(g, inv, den);
+    lam = tm_mul<false>(g, num, lam);
+    G1A r;
+    r.x = tm_sqr<true>(g, lam);
+    Fp d = fp_zero();
+    if (active) {
+        const Fp ax = a.x();
+        r.x = fp_sub(fp_sub(r.x, ax), b.x());
+        d = fp_sub(ax, r.x);
+    }
+    r.y = tm_mul<true>(g, lam, d);
+    if (active) {
+        r.y = fp_sub(r.y, a.y());
+        if (kind >= 2) { // rare: infinity on a side, or a point and its negative
+            r = G1A{fp_zero(), fp_zero()};
+            if (kind == 2) r = a.point();
+            if (kind == 3) r = b.point();
+        }
+        st_vec(out, r);
+    }
 }
 
 // A round's input and output lists, apart from the phase's other arguments:
@@ -624,34 +706,6 @@ struct RoundIO {
     const G1A *src;
     G1A *dst;
 };
-
-template <bool FIRST>
-__device__ __forceinline__ G1A flat_load(const FlatArgs &a, RoundIO io, uint32_t o, uint32_t t, uint32_t m) {
-    if (FIRST) {
-        const int v = a.dig[(size_t)o * a.L + t];
-        G1A pt;
-        if (v == 0) {
-            pt.x = fp_zero();
-            pt.y = fp_zero();
-            return pt;
-        }
-        pt = ldg_vec(comb_at(a.comb, comb_index(a, o, t, v)));
-        if (v < 0) pt.y = fp_neg(pt.y);
-        return pt;
-    }
-    return ld_vec(&io.src[(size_t)o * m + t]);
-}
-
-// the x coordinate of flat_load's point (0 for a zero digit)
-template <bool FIRST>
-__device__ __forceinline__ Fp flat_load_x(const FlatArgs &a, RoundIO io, uint32_t o, uint32_t t, uint32_t m) {
-    if (FIRST) {
-        const int v = a.dig[(size_t)o * a.L + t];
-        if (v == 0) return fp_zero();
-        return ldg_vec(&comb_at(a.comb, comb_index(a, o, t, v))->x);
-    }
-    return ld_vec(&io.src[(size_t)o * m + t].x);
-}
 
 // Signed digits of every scalar in the table's windows (window k: width w_k
 // at bit b_k, digits in (-2^(w_k - 1), 2^(w_k - 1)]; the top window takes the
@@ -718,20 +772,6 @@ __device__ __forceinline__ void pair_step_down(uint32_t &o, uint32_t &i, uint32_
 // cp.async while it computes the current pair.  The staging is chunk-major,
 // [buffer][16-byte chunk][thread], so a warp's reads of one chunk are one
 // contiguous 512-byte run (no bank conflicts).
-#ifndef VKZG_GATHER_PREFETCH
-#define VKZG_GATHER_PREFETCH 1
-#endif
-constexpr bool kGatherPrefetch = VKZG_GATHER_PREFETCH != 0;
-// the same staging in the later rounds, from the round's input lists (a build
-// switch, off: their pairs are coalesced runs of lists that stay largely in
-// L2, and staged they measured slower, phase A 12.04 against 11.84 ms at 256
-// blobs and 18 windows)
-#ifndef VKZG_LIST_PREFETCH
-#define VKZG_LIST_PREFETCH 0
-#endif
-constexpr bool kListPrefetch = kGatherPrefetch && VKZG_LIST_PREFETCH != 0;
-template <bool FIRST>
-constexpr bool kStaged = FIRST ? kGatherPrefetch : kListPrefetch;
 constexpr int kStageChunks = 12; // two 96-byte points
 constexpr size_t kStage1Bytes = 2 * 6 * kFlatThreads * sizeof(uint4);            // pass 1: x coordinates
 constexpr size_t kStage2Bytes = 2 * kStageChunks * kFlatThreads * sizeof(uint4); // pass 2: whole points
@@ -751,10 +791,50 @@ __device__ __forceinline__ const uint4 *comb_entry(const FlatArgs &a, uint32_t o
     return reinterpret_cast<const uint4 *>(comb_at(a.comb, comb_index(a, o, t, v)));
 }
 
-// pass 1 with the x coordinates of each pair staged one pair ahead, from the
-// digit table (FIRST) or from the round's input lists
+// point t of list o of a round
 template <bool FIRST>
-__device__ __forceinline__ void flat_pass1_staged(const FlatArgs &a, RoundIO io, uint32_t m, uint32_t gl, uint32_t NL) {
+__device__ __forceinline__ PointRef flat_ref(const FlatArgs &a, RoundIO io, uint32_t o, uint32_t t, uint32_t m) {
+    if (FIRST) {
+        const int v = a.dig[(size_t)o * a.L + t];
+        return PointRef{v ? comb_at(a.comb, comb_index(a, o, t, v)) : nullptr, v < 0};
+    }
+    return PointRef{&io.src[(size_t)o * m + t], false};
+}
+
+// a staged point: chunk c of thread t at w[c * kFlatThreads]; v its digit (0:
+// infinity, negative: sign flipped)
+struct StagedRef {
+    const uint4 *w;
+    int v;
+    __device__ __forceinline__ Fp part(int c0) const {
+        Fp x;
+        uint4 *d = reinterpret_cast<uint4 *>(&x);
+#pragma unroll
+        for (int c = 0; c < 3; c++) d[c] = w[(c0 + c) * kFlatThreads];
+        return x;
+    }
+    __device__ __forceinline__ Fp x() const { return v ? part(0) : fp_zero(); }
+    __device__ __forceinline__ Fp y() const {
+        if (!v) return fp_zero();
+        const Fp y = part(3);
+        return v < 0 ? fp_neg(y) : y;
+    }
+    __device__ __forceinline__ G1A point() const { return G1A{x(), y()}; }
+};
+// pass 1 stages x alone: where a pair needs the whole point, from the table
+struct StagedXRef {
+    StagedRef s;
+    const FlatArgs &a;
+    RoundIO io;
+    uint32_t o, t, m;
+    __device__ __forceinline__ Fp x() const { return s.x(); }
+    __device__ __forceinline__ G1A point() const { return flat_ref<true>(a, io, o, t, m).point(); }
+};
+
+// pass 1 with the x coordinates of each pair staged one pair ahead from the digit table
+template <class G>
+__device__ __forceinline__ void flat_pass1_staged(G &g, const FlatArgs &a, RoundIO io, uint32_t m, uint32_t gl,
+                                                  uint32_t NL) {
     extern __shared__ uint4 stage[];
     uint4 *my = stage + threadIdx.x; // chunk c of buffer b: my[(b * 6 + c) * kFlatThreads]
     const uint32_t wg = gl >> 5;
@@ -763,63 +843,52 @@ __device__ __forceinline__ void flat_pass1_staged(const FlatArgs &a, RoundIO io,
     const uint32_t dq = NL / h, dr = NL % h;
     uint32_t *pre = a.pre + (size_t)wg * a.slots * 384;
     auto issue = [&](int b, uint32_t o, uint32_t i, int &v0, int &v1) {
-        if constexpr (FIRST) {
-            const int16_t *d = a.dig + (size_t)o * a.L + 2 * i;
-            v0 = d[0];
-            v1 = d[1];
-            if (v0) {
-                const uint4 *src = comb_entry(a, o, 2 * i, v0);
-                for (int c = 0; c < 3; c++) cp_async16(&my[(b * 6 + c) * kFlatThreads], src + c);
-            }
-            if (v1) {
-                const uint4 *src = comb_entry(a, o, 2 * i + 1, v1);
-                for (int c = 0; c < 3; c++) cp_async16(&my[(b * 6 + 3 + c) * kFlatThreads], src + c);
-            }
-        } else {
-            v0 = v1 = 1; // list points are stored whole, infinity as (0, 0)
-            const uint4 *src = reinterpret_cast<const uint4 *>(&io.src[(size_t)o * m + 2 * i]);
+        const int16_t *d = a.dig + (size_t)o * a.L + 2 * i;
+        v0 = d[0];
+        v1 = d[1];
+        if (v0) {
+            const uint4 *src = comb_entry(a, o, 2 * i, v0);
             for (int c = 0; c < 3; c++) cp_async16(&my[(b * 6 + c) * kFlatThreads], src + c);
-            for (int c = 0; c < 3; c++) cp_async16(&my[(b * 6 + 3 + c) * kFlatThreads], src + 6 + c);
+        }
+        if (v1) {
+            const uint4 *src = comb_entry(a, o, 2 * i + 1, v1);
+            for (int c = 0; c < 3; c++) cp_async16(&my[(b * 6 + 3 + c) * kFlatThreads], src + c);
         }
         cp_async_commit();
     };
-    auto x_of = [&](int b, int half, int v) {
-        Fp x;
-        if (v == 0) return fp_zero();
-        uint4 *w = reinterpret_cast<uint4 *>(&x);
-        for (int c = 0; c < 3; c++) w[c] = my[(b * 6 + 3 * half + c) * kFlatThreads];
-        return x;
-    };
     Fp acc = fp_one();
-    int s = 0, v0 = 0, v1 = 0;
+    int v0 = 0, v1 = 0;
     uint32_t o = gl / h, i = gl % h;
     if (gl < P) issue(0, o, i, v0, v1);
-    for (uint32_t p = gl; p < P; p += NL, s++) {
+    const int S = group_steps(P, gl, NL);
+    uint32_t p = gl;
+    for (int s = 0; s < S; s++, p += NL) {
+        const bool active = p < P;
         uint32_t on = o, in = i;
         int w0 = 0, w1 = 0;
-        if (p + NL < P) {
+        if (active && p + NL < P) {
             pair_step_up(on, in, h, dq, dr);
             issue((s + 1) & 1, on, in, w0, w1);
             cp_async_wait<1>();
         } else {
             cp_async_wait<0>();
         }
-        const Fp x = x_of(s & 1, 0, v0), y = x_of(s & 1, 1, v1);
-        wb_store_pre(pre, s, acc);
-        acc = fp_mul(acc, pair_denominator_x(x, y, [&] { return flat_load<FIRST>(a, io, o, 2 * i, m); },
-                                             [&] { return flat_load<FIRST>(a, io, o, 2 * i + 1, m); }));
+        const uint4 *w = my + (s & 1) * 6 * kFlatThreads;
+        pass1_pair(g, acc, active, pre, s, StagedXRef{StagedRef{w, v0}, a, io, o, 2 * i, m},
+                   StagedXRef{StagedRef{w + 3 * kFlatThreads, v1}, a, io, o, 2 * i + 1, m});
         o = on;
         i = in;
         v0 = w0;
         v1 = w1;
     }
-    flat_pass1_products(acc, a.others, a.tot, gl, wg);
+    flat_pass1_products(g, acc, a.others, a.tot, gl, wg);
 }
 
-template <bool FIRST>
-__device__ __forceinline__ void flat_pass1_body(const FlatArgs &a, RoundIO io, uint32_t m, uint32_t gl, uint32_t NL) {
-    if constexpr (kStaged<FIRST>) {
-        flat_pass1_staged<FIRST>(a, io, m, gl, NL);
+template <bool FIRST, class G>
+__device__ __forceinline__ void flat_pass1_body(G &g, const FlatArgs &a, RoundIO io, uint32_t m, uint32_t gl,
+                                                uint32_t NL) {
+    if constexpr (FIRST) {
+        flat_pass1_staged(g, a, io, m, gl, NL);
         return;
     }
     const uint32_t wg = gl >> 5;
@@ -828,21 +897,23 @@ __device__ __forceinline__ void flat_pass1_body(const FlatArgs &a, RoundIO io, u
     const uint32_t dq = NL / h, dr = NL % h;
     uint32_t *pre = a.pre + (size_t)wg * a.slots * 384;
     Fp acc = fp_one();
-    int s = 0;
     uint32_t o = gl / h, i = gl % h;
-    for (uint32_t p = gl; p < P; p += NL, s++) {
-        const Fp x = flat_load_x<FIRST>(a, io, o, 2 * i, m), y = flat_load_x<FIRST>(a, io, o, 2 * i + 1, m);
-        wb_store_pre(pre, s, acc);
-        acc = fp_mul(acc, pair_denominator_x(x, y, [&] { return flat_load<FIRST>(a, io, o, 2 * i, m); },
-                                             [&] { return flat_load<FIRST>(a, io, o, 2 * i + 1, m); }));
+    const int S = group_steps(P, gl, NL);
+    uint32_t p = gl;
+    for (int s = 0; s < S; s++, p += NL) {
+        pass1_pair(g, acc, p < P, pre, s, flat_ref<false>(a, io, o, 2 * i, m), flat_ref<false>(a, io, o, 2 * i + 1, m));
         pair_step_up(o, i, h, dq, dr);
     }
-    flat_pass1_products(acc, a.others, a.tot, gl, wg);
+    flat_pass1_products(g, acc, a.others, a.tot, gl, wg);
 }
 
 template <bool FIRST>
 __global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSM) k_flat_pass1(FlatArgs a, uint32_t m) {
-    flat_pass1_body<FIRST>(a, RoundIO{a.src, a.dst}, m, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    __shared__ __align__(128) uint8_t tm_area[kTmSmem];
+    Tm g = tm_begin(tm_area);
+    flat_pass1_body<FIRST>(g, a, RoundIO{a.src, a.dst}, m, blockIdx.x * blockDim.x + threadIdx.x,
+                           gridDim.x * blockDim.x);
+    tm_end(tm_area, a.err, a.n_err);
 }
 
 // Inverts the n warp products, each by the four lanes of a quad (fp_inv_quad,
@@ -868,17 +939,18 @@ static void launch_flat_invert(const Fp *tot, Fp *totinv, int n, cudaStream_t s)
     k_flat_invert<<<(4 * n + kInvThreads - 1) / kInvThreads, kInvThreads, 0, s>>>(tot, totinv, n);
 }
 
-// Products inlined into this loop instead of called: measured 14.1 against
-// 13.1 ms of phase A at 256 blobs (the loop body outgrows the instruction
-// cache), so the calls stay.
-#ifndef VKZG_PASS2_INLINE
-#define VKZG_PASS2_INLINE 0
-#endif
-constexpr bool kPass2Inline = VKZG_PASS2_INLINE != 0;
-// pass 2 with the two points of each pair staged one pair ahead, from the
-// digit table (FIRST) or from the round's input lists
+// an odd list's last point moves up unchanged
 template <bool FIRST>
-__device__ __forceinline__ void flat_pass2_staged(const FlatArgs &a, RoundIO io, uint32_t m, uint32_t gl, uint32_t NL) {
+__device__ __forceinline__ void flat_odd_points(const FlatArgs &a, RoundIO io, uint32_t m, uint32_t gl, uint32_t NL) {
+    if (!(m & 1u)) return;
+    for (uint32_t l = gl; l < (uint32_t)a.n_lists; l += NL)
+        st_vec(&io.dst[(size_t)l * ((m + 1) >> 1) + (m >> 1)], flat_ref<FIRST>(a, io, l, m - 1, m).point());
+}
+
+// pass 2 with the two points of each pair staged one pair ahead from the digit table
+template <class G>
+__device__ __forceinline__ void flat_pass2_staged(G &g, const FlatArgs &a, RoundIO io, uint32_t m, uint32_t gl,
+                                                  uint32_t NL) {
     extern __shared__ uint4 stage[];
     uint4 *my = stage + threadIdx.x; // chunk c of buffer b: my[(b * kStageChunks + c) * kFlatThreads]
     const uint32_t wg = gl >> 5;
@@ -886,78 +958,58 @@ __device__ __forceinline__ void flat_pass2_staged(const FlatArgs &a, RoundIO io,
     const uint32_t P = (uint32_t)a.n_lists * h;
     const uint32_t dq = NL / h, dr = NL % h;
     const uint32_t *pre = a.pre + (size_t)wg * a.slots * 384;
-    Fp inv = fp_mul(ld_vec(&a.totinv[wg]), ld_vec(&a.others[gl]));
-    const int S = P > gl ? (int)((P - gl + NL - 1) / NL) : 0;
     auto issue = [&](int b, uint32_t o, uint32_t i, int &v0, int &v1) {
-        if constexpr (FIRST) {
-            const int16_t *d = a.dig + (size_t)o * a.L + 2 * i;
-            v0 = d[0];
-            v1 = d[1];
-            if (v0) {
-                const uint4 *src = comb_entry(a, o, 2 * i, v0);
-                for (int c = 0; c < 6; c++) cp_async16(&my[(b * kStageChunks + c) * kFlatThreads], src + c);
-            }
-            if (v1) {
-                const uint4 *src = comb_entry(a, o, 2 * i + 1, v1);
-                for (int c = 0; c < 6; c++) cp_async16(&my[(b * kStageChunks + 6 + c) * kFlatThreads], src + c);
-            }
-        } else {
-            v0 = v1 = 1; // the pair's two points, 192 contiguous bytes of the list
-            const uint4 *src = reinterpret_cast<const uint4 *>(&io.src[(size_t)o * m + 2 * i]);
-            for (int c = 0; c < kStageChunks; c++) cp_async16(&my[(b * kStageChunks + c) * kFlatThreads], src + c);
+        const int16_t *d = a.dig + (size_t)o * a.L + 2 * i;
+        v0 = d[0];
+        v1 = d[1];
+        if (v0) {
+            const uint4 *src = comb_entry(a, o, 2 * i, v0);
+            for (int c = 0; c < 6; c++) cp_async16(&my[(b * kStageChunks + c) * kFlatThreads], src + c);
+        }
+        if (v1) {
+            const uint4 *src = comb_entry(a, o, 2 * i + 1, v1);
+            for (int c = 0; c < 6; c++) cp_async16(&my[(b * kStageChunks + 6 + c) * kFlatThreads], src + c);
         }
         cp_async_commit();
     };
-    auto point = [&](int b, int half, int v) {
-        G1A pt;
-        if (v == 0) {
-            pt.x = fp_zero();
-            pt.y = fp_zero();
-            return pt;
-        }
-        uint4 *w = reinterpret_cast<uint4 *>(&pt);
-        for (int c = 0; c < 6; c++) w[c] = my[(b * kStageChunks + 6 * half + c) * kFlatThreads];
-        if (v < 0) pt.y = fp_neg(pt.y);
-        return pt;
-    };
+    const int S = group_steps(P, gl, NL);
+    const int own = P > gl ? (int)((P - gl + NL - 1) / NL) : 0; // S or S - 1
     uint32_t o = 0, i = 0;
     int v0 = 0, v1 = 0;
-    if (S > 0) {
-        const uint32_t p_last = gl + (uint32_t)(S - 1) * NL;
+    if (own > 0) {
+        const uint32_t p_last = gl + (uint32_t)(own - 1) * NL;
         o = p_last / h;
         i = p_last % h;
-        issue((S - 1) & 1, o, i, v0, v1);
+        issue((own - 1) & 1, o, i, v0, v1);
     }
+    Fp inv = tm_mul<false>(g, ld_vec(&a.totinv[wg]), ld_vec(&a.others[gl]));
     for (int t = S - 1; t >= 0; t--) {
+        const bool active = t < own;
         uint32_t on = o, in = i;
-        int w0 = 0, w1 = 0;
-        if (t > 0) {
+        int w0 = v0, w1 = v1;
+        if (active && t > 0) {
             pair_step_down(on, in, h, dq, dr);
             issue((t - 1) & 1, on, in, w0, w1);
             cp_async_wait<1>();
-        } else {
+        } else if (active) {
             cp_async_wait<0>();
         }
-        const G1A x = point(t & 1, 0, v0), y = point(t & 1, 1, v1);
-        const int kind = pair_kind(x, y);
-        const Fp den = pair_denominator(x, y, kind);
-        const Fp inv_den = pmul<kPass2Inline>(inv, wb_load_pre(pre, t));
-        inv = pmul<kPass2Inline>(inv, den);
-        st_vec(&io.dst[(size_t)o * m_next + i], pair_result<kPass2Inline>(x, y, kind, inv_den));
+        const uint4 *w = my + (t & 1) * kStageChunks * kFlatThreads;
+        pass2_pair(g, inv, active, pre, t, StagedRef{w, v0}, StagedRef{w + 6 * kFlatThreads, v1},
+                   &io.dst[(size_t)o * m_next + i]);
         o = on;
         i = in;
         v0 = w0;
         v1 = w1;
     }
-    if (m & 1u)
-        for (uint32_t l = gl; l < (uint32_t)a.n_lists; l += NL)
-            st_vec(&io.dst[(size_t)l * m_next + h], flat_load<FIRST>(a, io, l, m - 1, m));
+    flat_odd_points<true>(a, io, m, gl, NL);
 }
 
-template <bool FIRST>
-__device__ __forceinline__ void flat_pass2_body(const FlatArgs &a, RoundIO io, uint32_t m, uint32_t gl, uint32_t NL) {
-    if constexpr (kStaged<FIRST>) {
-        flat_pass2_staged<FIRST>(a, io, m, gl, NL);
+template <bool FIRST, class G>
+__device__ __forceinline__ void flat_pass2_body(G &g, const FlatArgs &a, RoundIO io, uint32_t m, uint32_t gl,
+                                                uint32_t NL) {
+    if constexpr (FIRST) {
+        flat_pass2_staged(g, a, io, m, gl, NL);
         return;
     }
     const uint32_t wg = gl >> 5;
@@ -965,31 +1017,30 @@ __device__ __forceinline__ void flat_pass2_body(const FlatArgs &a, RoundIO io, u
     const uint32_t P = (uint32_t)a.n_lists * h;
     const uint32_t dq = NL / h, dr = NL % h;
     const uint32_t *pre = a.pre + (size_t)wg * a.slots * 384;
-    Fp inv = fp_mul(ld_vec(&a.totinv[wg]), ld_vec(&a.others[gl]));
-    const int S = P > gl ? (int)((P - gl + NL - 1) / NL) : 0;
+    Fp inv = tm_mul<false>(g, ld_vec(&a.totinv[wg]), ld_vec(&a.others[gl]));
+    const int S = group_steps(P, gl, NL);
+    const int own = P > gl ? (int)((P - gl + NL - 1) / NL) : 0; // S or S - 1
     uint32_t o = 0, i = 0;
-    if (S > 0) {
-        const uint32_t p_last = gl + (uint32_t)(S - 1) * NL;
+    if (own > 0) {
+        const uint32_t p_last = gl + (uint32_t)(own - 1) * NL;
         o = p_last / h;
         i = p_last % h;
     }
     for (int t = S - 1; t >= 0; t--) {
-        if (t < S - 1) pair_step_down(o, i, h, dq, dr);
-        const G1A x = flat_load<FIRST>(a, io, o, 2 * i, m), y = flat_load<FIRST>(a, io, o, 2 * i + 1, m);
-        const int kind = pair_kind(x, y);
-        const Fp den = pair_denominator(x, y, kind);
-        const Fp inv_den = pmul<kPass2Inline>(inv, wb_load_pre(pre, t));
-        inv = pmul<kPass2Inline>(inv, den);
-        st_vec(&io.dst[(size_t)o * m_next + i], pair_result<kPass2Inline>(x, y, kind, inv_den));
+        pass2_pair(g, inv, t < own, pre, t, flat_ref<false>(a, io, o, 2 * i, m), flat_ref<false>(a, io, o, 2 * i + 1, m),
+                   &io.dst[(size_t)o * m_next + i]);
+        if (t < own && t > 0) pair_step_down(o, i, h, dq, dr);
     }
-    if (m & 1u)
-        for (uint32_t l = gl; l < (uint32_t)a.n_lists; l += NL)
-            st_vec(&io.dst[(size_t)l * m_next + h], flat_load<FIRST>(a, io, l, m - 1, m));
+    flat_odd_points<false>(a, io, m, gl, NL);
 }
 
 template <bool FIRST>
 __global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSM) k_flat_pass2(FlatArgs a, uint32_t m) {
-    flat_pass2_body<FIRST>(a, RoundIO{a.src, a.dst}, m, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    __shared__ __align__(128) uint8_t tm_area[kTmSmem];
+    Tm g = tm_begin(tm_area);
+    flat_pass2_body<FIRST>(g, a, RoundIO{a.src, a.dst}, m, blockIdx.x * blockDim.x + threadIdx.x,
+                           gridDim.x * blockDim.x);
+    tm_end(tm_area, a.err, a.n_err);
 }
 
 // The last m <= kTreeTail points of each list (affine, left by the tree
@@ -1057,11 +1108,11 @@ const G1A *run_tree_rounds(FlatArgs a, const G1A *first_src, uint32_t *m_io, uin
     while (m > stop) {
         a.src = cur;
         a.dst = bufs[out];
-        if (first) k_flat_pass1<FIRST><<<blocks, kFlatThreads, kStaged<FIRST> ? kStage1Bytes : 0, s>>>(a, m);
-        else k_flat_pass1<false><<<blocks, kFlatThreads, kStaged<false> ? kStage1Bytes : 0, s>>>(a, m);
+        if (first) k_flat_pass1<FIRST><<<blocks, kFlatThreads, FIRST ? kStage1Bytes : 0, s>>>(a, m);
+        else k_flat_pass1<false><<<blocks, kFlatThreads, 0, s>>>(a, m);
         launch_flat_invert(a.tot, a.totinv, warps, s);
-        if (first) k_flat_pass2<FIRST><<<blocks, kFlatThreads, kStaged<FIRST> ? kStage2Bytes : 0, s>>>(a, m);
-        else k_flat_pass2<false><<<blocks, kFlatThreads, kStaged<false> ? kStage2Bytes : 0, s>>>(a, m);
+        if (first) k_flat_pass2<FIRST><<<blocks, kFlatThreads, FIRST ? kStage2Bytes : 0, s>>>(a, m);
+        else k_flat_pass2<false><<<blocks, kFlatThreads, 0, s>>>(a, m);
         *launched += 3;
         cur = bufs[out];
         out ^= 1;
@@ -1070,15 +1121,6 @@ const G1A *run_tree_rounds(FlatArgs a, const G1A *first_src, uint32_t *m_io, uin
     }
     *m_io = m;
     return cur;
-}
-
-// The later rounds' pass kernels stage their pairs in dynamic shared memory.
-static cudaError_t configure_list_rounds() {
-    if (!kListPrefetch) return cudaSuccess;
-    cudaError_t e =
-        cudaFuncSetAttribute(k_flat_pass1<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStage1Bytes);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_flat_pass2<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStage2Bytes);
 }
 
 // Sums of n_lists lists of m points (list o at lists[o m ..]) by the same
@@ -1095,7 +1137,6 @@ int launch_tree_sums(const G1A *lists, int n_lists, uint32_t m, G1A *buf0, G1A *
     a.slots = slots;
     a.n_lists = n_lists;
     int launched = 0;
-    if (configure_list_rounds() != cudaSuccess) return 0;
     const G1A *res = run_tree_rounds<false>(a, lists, &m, 1, buf0, buf1, blocks, s, &launched);
     cudaMemcpyAsync(sums, res, (size_t)n_lists * sizeof(G1A), cudaMemcpyDeviceToDevice, s);
     count_launches(launched);
@@ -1114,12 +1155,12 @@ int launch_tree_sums(const G1A *lists, int n_lists, uint32_t m, G1A *buf0, G1A *
 #define VKZG_COOP_FN __device__ __forceinline__
 #endif
 template <bool FIRST>
-VKZG_COOP_FN void coop_flat_pass1(FlatArgs a, RoundIO io, uint32_t m, uint32_t gl, uint32_t NL) {
-    flat_pass1_body<FIRST>(a, io, m, gl, NL);
+VKZG_COOP_FN void coop_flat_pass1(ScalarMul &t, FlatArgs a, RoundIO io, uint32_t m, uint32_t gl, uint32_t NL) {
+    flat_pass1_body<FIRST>(t, a, io, m, gl, NL);
 }
 template <bool FIRST>
-VKZG_COOP_FN void coop_flat_pass2(FlatArgs a, RoundIO io, uint32_t m, uint32_t gl, uint32_t NL) {
-    flat_pass2_body<FIRST>(a, io, m, gl, NL);
+VKZG_COOP_FN void coop_flat_pass2(ScalarMul &t, FlatArgs a, RoundIO io, uint32_t m, uint32_t gl, uint32_t NL) {
+    flat_pass2_body<FIRST>(t, a, io, m, gl, NL);
 }
 
 // The inversions between the passes of a cooperative round: one warp in 32
@@ -1134,13 +1175,17 @@ __device__ __noinline__ void coop_invert(const Fp *tot, Fp *totinv, uint32_t n, 
     if (t < n) st_vec(&totinv[t], fp_inv_fast(ld_vec(&tot[t])));
 }
 
+// The cooperative kernels make their products with the scalar multiplier: a
+// cooperative launch of a kernel that allocates TMEM is granted one block per
+// SM only (the driver's occupancy count for it is one), and their grid is two.
+//
 // Cooperative form of run_tree_rounds: every round of the tree in one launch,
 // the passes and the inversion between them separated by grid barriers.  The
 // phase's arguments stay in the kernel's parameters (only the round's lists
 // change from round to round), so the passes compile as in their own kernels.
 template <bool FIRST>
-__global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSM) k_coop_tree(FlatArgs a, const G1A *first_src, G1A *buf0,
-                                                               G1A *buf1, uint32_t m, uint32_t stop, GridSync g) {
+__device__ __forceinline__ void coop_tree(ScalarMul &t, FlatArgs a, const G1A *first_src, G1A *buf0, G1A *buf1, uint32_t m,
+                                          uint32_t stop, GridSync g) {
     const uint32_t gl = blockIdx.x * blockDim.x + threadIdx.x, NL = gridDim.x * blockDim.x;
     RoundIO io{first_src, buf0};
     if constexpr (FIRST) {
@@ -1161,24 +1206,30 @@ __global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSM) k_coop_tree(Fl
             }
         }
         if (!grid_sync(g)) return;
-        coop_flat_pass1<true>(a, io, m, gl, NL);
+        coop_flat_pass1<true>(t, a, io, m, gl, NL);
         if (!grid_sync(g)) return;
         coop_invert(a.tot, a.totinv, NL >> 5, gl, NL);
         if (!grid_sync(g)) return;
-        coop_flat_pass2<true>(a, io, m, gl, NL);
+        coop_flat_pass2<true>(t, a, io, m, gl, NL);
     } else {
         while (m > stop) {
-            coop_flat_pass1<false>(a, io, m, gl, NL);
+            coop_flat_pass1<false>(t, a, io, m, gl, NL);
             if (!grid_sync(g)) return;
             coop_invert(a.tot, a.totinv, NL >> 5, gl, NL);
             if (!grid_sync(g)) return;
-            coop_flat_pass2<false>(a, io, m, gl, NL);
+            coop_flat_pass2<false>(t, a, io, m, gl, NL);
             io.src = io.dst;
             io.dst = io.dst == buf0 ? buf1 : buf0;
             m = (m + 1) >> 1;
             if (m > stop && !grid_sync(g)) return;
         }
     }
+}
+template <bool FIRST>
+__global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSM) k_coop_tree(FlatArgs a, const G1A *first_src, G1A *buf0,
+                                                               G1A *buf1, uint32_t m, uint32_t stop, GridSync g) {
+    ScalarMul t;
+    coop_tree<FIRST>(t, a, first_src, buf0, buf1, m, stop, g);
 }
 
 // the buffer holding the lists after run_tree_rounds' rounds from m down to stop
@@ -1245,6 +1296,8 @@ int launch_phase_a_flat(const ProofWork &w, int n, cudaStream_t s) {
     a.totinv = w.flat_totinv;
     a.slots = w.flat_slots;
     a.n_lists = lists;
+    a.err = w.err;
+    a.n_err = (uint32_t)n;
     int launched = 0;
     uint32_t m = (uint32_t)L;
     const G1A *res;
@@ -1340,6 +1393,7 @@ struct FlatBArgs {
     Fp *others, *tot, *totinv;
     size_t slots;
     int n_blobs;
+    uint32_t *err; // error words, one per blob
 };
 
 // shared copy of one round's plan (and, in round 0, the tap items)
@@ -1403,30 +1457,17 @@ __device__ __forceinline__ const G1A *flatb_src(const FlatBArgs &a, const FlatBR
 
 // element e of bucket k of output o (part q)
 template <bool FIRST>
-__device__ __forceinline__ G1A flatb_load(const FlatBArgs &a, RoundIO io, const FlatBRound &sr, const uint32_t *items,
-                                          const uint32_t *offs, uint32_t o, int q, int k, uint32_t e) {
+__device__ __forceinline__ PointRef flatb_ref(const FlatBArgs &a, RoundIO io, const FlatBRound &sr,
+                                              const uint32_t *items, const uint32_t *offs, uint32_t o, int q, int k,
+                                              uint32_t e) {
     if (FIRST) {
         const uint32_t packed = items[kDigits * sr.off[q] + offs[q * (kBuckets + 1) + k] + e];
         const int tap = (int)(packed & 0xffu), d = (int)((packed >> 8) & 0xffu);
         const uint32_t b = o / kCells, aa = o % kCells - sr.off[q];
-        G1A pt = ld_vec(flatb_src(a, sr, b, q, (aa - (uint32_t)tap) & (sr.size[q] - 1), d));
-        if (((packed >> 16) & 1u) != (sr.nega[q] && tap > (int)aa)) pt.y = fp_neg(pt.y);
-        return pt;
+        return PointRef{flatb_src(a, sr, b, q, (aa - (uint32_t)tap) & (sr.size[q] - 1), d),
+                        ((packed >> 16) & 1u) != (sr.nega[q] && tap > (int)aa)};
     }
-    return ld_vec(&io.src[(size_t)o * sr.stride + sr.base[q][k] + e]);
-}
-
-// the x coordinate of flatb_load's point
-template <bool FIRST>
-__device__ __forceinline__ Fp flatb_load_x(const FlatBArgs &a, RoundIO io, const FlatBRound &sr, const uint32_t *items,
-                                           const uint32_t *offs, uint32_t o, int q, int k, uint32_t e) {
-    if (FIRST) {
-        const uint32_t packed = items[kDigits * sr.off[q] + offs[q * (kBuckets + 1) + k] + e];
-        const int tap = (int)(packed & 0xffu), d = (int)((packed >> 8) & 0xffu);
-        const uint32_t b = o / kCells, aa = o % kCells - sr.off[q];
-        return ld_vec(&flatb_src(a, sr, b, q, (aa - (uint32_t)tap) & (sr.size[q] - 1), d)->x);
-    }
-    return ld_vec(&io.src[(size_t)o * sr.stride + sr.base[q][k] + e].x);
+    return PointRef{&io.src[(size_t)o * sr.stride + sr.base[q][k] + e], false};
 }
 
 // pair p of the round -> output, part, bucket, index
@@ -1443,9 +1484,9 @@ __device__ __forceinline__ void flatb_pair(const FlatBRound &sr, uint32_t p, uin
     i = r - sr.pscan[q][k];
 }
 
-template <bool FIRST>
-__device__ __forceinline__ void flatb_pass1_body(const FlatBArgs &a, RoundIO io, int r, uint4 *dyn_smem, uint32_t gl,
-                                                 uint32_t NL) {
+template <bool FIRST, class G>
+__device__ __forceinline__ void flatb_pass1_body(G &g, const FlatBArgs &a, RoundIO io, int r, uint4 *dyn_smem,
+                                                 uint32_t gl, uint32_t NL) {
     FlatBRound &sr = *reinterpret_cast<FlatBRound *>(dyn_smem);
     uint32_t *items = reinterpret_cast<uint32_t *>(&sr + 1), *offs = items + kPartItemsMax;
     flatb_stage<FIRST>(a, r, sr, items, offs);
@@ -1453,30 +1494,35 @@ __device__ __forceinline__ void flatb_pass1_body(const FlatBArgs &a, RoundIO io,
     const uint32_t P = sr.pair_end[sr.n_parts - 1];
     uint32_t *pre = a.pre + (size_t)wg * a.slots * 384;
     Fp acc = fp_one();
-    int s = 0;
-    for (uint32_t p = gl; p < P; p += NL, s++) {
-        uint32_t o, i;
-        int q, k;
-        flatb_pair(sr, p, o, q, k, i);
-        const Fp x = flatb_load_x<FIRST>(a, io, sr, items, offs, o, q, k, 2 * i);
-        const Fp y = flatb_load_x<FIRST>(a, io, sr, items, offs, o, q, k, 2 * i + 1);
-        wb_store_pre(pre, s, acc);
-        acc = fp_mul(acc, pair_denominator_x(x, y, [&] { return flatb_load<FIRST>(a, io, sr, items, offs, o, q, k, 2 * i); },
-                                             [&] { return flatb_load<FIRST>(a, io, sr, items, offs, o, q, k, 2 * i + 1); }));
+    const int S = group_steps(P, gl, NL);
+    uint32_t p = gl;
+    for (int s = 0; s < S; s++, p += NL) {
+        PointRef x{nullptr, false}, y = x;
+        if (p < P) {
+            uint32_t o, i;
+            int q, k;
+            flatb_pair(sr, p, o, q, k, i);
+            x = flatb_ref<FIRST>(a, io, sr, items, offs, o, q, k, 2 * i);
+            y = flatb_ref<FIRST>(a, io, sr, items, offs, o, q, k, 2 * i + 1);
+        }
+        pass1_pair(g, acc, p < P, pre, s, x, y);
     }
-    flat_pass1_products(acc, a.others, a.tot, gl, wg);
+    flat_pass1_products(g, acc, a.others, a.tot, gl, wg);
 }
 
 template <bool FIRST>
 __global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSM) k_flatb_pass1(FlatBArgs a, int r) {
     extern __shared__ uint4 dyn_smem[];
-    flatb_pass1_body<FIRST>(a, RoundIO{a.src, a.dst}, r, dyn_smem, blockIdx.x * blockDim.x + threadIdx.x,
+    __shared__ __align__(128) uint8_t tm_area[kTmSmem];
+    Tm g = tm_begin(tm_area);
+    flatb_pass1_body<FIRST>(g, a, RoundIO{a.src, a.dst}, r, dyn_smem, blockIdx.x * blockDim.x + threadIdx.x,
                             gridDim.x * blockDim.x);
+    tm_end(tm_area, a.err, (uint32_t)a.n_blobs);
 }
 
-template <bool FIRST>
-__device__ __forceinline__ void flatb_pass2_body(const FlatBArgs &a, RoundIO io, int r, uint4 *dyn_smem, uint32_t gl,
-                                                 uint32_t NL) {
+template <bool FIRST, class G>
+__device__ __forceinline__ void flatb_pass2_body(G &g, const FlatBArgs &a, RoundIO io, int r, uint4 *dyn_smem,
+                                                 uint32_t gl, uint32_t NL) {
     FlatBRound &sr = *reinterpret_cast<FlatBRound *>(dyn_smem);
     uint32_t *items = reinterpret_cast<uint32_t *>(&sr + 1), *offs = items + kPartItemsMax;
     flatb_stage<FIRST>(a, r, sr, items, offs);
@@ -1484,21 +1530,21 @@ __device__ __forceinline__ void flatb_pass2_body(const FlatBArgs &a, RoundIO io,
     const uint32_t P = sr.pair_end[sr.n_parts - 1];
     const uint32_t *pre = a.pre + (size_t)wg * a.slots * 384;
     const bool last = r + 1 == a.plan->rounds;
-    Fp inv = fp_mul(ld_vec(&a.totinv[wg]), ld_vec(&a.others[gl]));
-    const int S = P > gl ? (int)((P - gl + NL - 1) / NL) : 0;
-    for (int t = S - 1; t >= 0; t--) {
+    Fp inv = tm_mul<false>(g, ld_vec(&a.totinv[wg]), ld_vec(&a.others[gl]));
+    for (int t = group_steps(P, gl, NL) - 1; t >= 0; t--) {
         const uint32_t p = gl + (uint32_t)t * NL;
-        uint32_t o, i;
-        int q, k;
-        flatb_pair(sr, p, o, q, k, i);
-        const G1A x = flatb_load<FIRST>(a, io, sr, items, offs, o, q, k, 2 * i);
-        const G1A y = flatb_load<FIRST>(a, io, sr, items, offs, o, q, k, 2 * i + 1);
-        const int kind = pair_kind(x, y);
-        const Fp den = pair_denominator(x, y, kind);
-        const Fp inv_den = fp_mul(inv, wb_load_pre(pre, t));
-        inv = fp_mul(inv, den);
-        G1A *d = last ? &a.bucket_aff[(size_t)o * kBuckets + k] : &io.dst[(size_t)o * sr.stride_next + sr.base_next[q][k] + i];
-        st_vec(d, pair_result(x, y, kind, inv_den));
+        PointRef x{nullptr, false}, y = x;
+        G1A *d = nullptr;
+        if (p < P) {
+            uint32_t o, i;
+            int q, k;
+            flatb_pair(sr, p, o, q, k, i);
+            x = flatb_ref<FIRST>(a, io, sr, items, offs, o, q, k, 2 * i);
+            y = flatb_ref<FIRST>(a, io, sr, items, offs, o, q, k, 2 * i + 1);
+            d = last ? &a.bucket_aff[(size_t)o * kBuckets + k]
+                     : &io.dst[(size_t)o * sr.stride_next + sr.base_next[q][k] + i];
+        }
+        pass2_pair(g, inv, p < P, pre, t, x, y, d);
     }
     // odd last elements move up unchanged
     const FlatBPlan &pl = *a.plan;
@@ -1517,7 +1563,7 @@ __device__ __forceinline__ void flatb_pass2_body(const FlatBArgs &a, RoundIO io,
             const uint32_t c = sr.cnt[q][k];
             G1A *d = last ? &a.bucket_aff[(size_t)o * kBuckets + k]
                           : &io.dst[(size_t)o * sr.stride_next + sr.base_next[q][k] + (c >> 1)];
-            st_vec(d, flatb_load<FIRST>(a, io, sr, items, offs, o, q, k, c - 1));
+            st_vec(d, flatb_ref<FIRST>(a, io, sr, items, offs, o, q, k, c - 1).point());
         }
         odd_begin += odd_q;
     }
@@ -1544,8 +1590,11 @@ __device__ __forceinline__ void flatb_pass2_body(const FlatBArgs &a, RoundIO io,
 template <bool FIRST>
 __global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSM) k_flatb_pass2(FlatBArgs a, int r) {
     extern __shared__ uint4 dyn_smem[];
-    flatb_pass2_body<FIRST>(a, RoundIO{a.src, a.dst}, r, dyn_smem, blockIdx.x * blockDim.x + threadIdx.x,
+    __shared__ __align__(128) uint8_t tm_area[kTmSmem];
+    Tm g = tm_begin(tm_area);
+    flatb_pass2_body<FIRST>(g, a, RoundIO{a.src, a.dst}, r, dyn_smem, blockIdx.x * blockDim.x + threadIdx.x,
                             gridDim.x * blockDim.x);
+    tm_end(tm_area, a.err, (uint32_t)a.n_blobs);
 }
 
 // The shared pair sums of phase B as one grid-wide round: point m of blob b is
@@ -1561,68 +1610,61 @@ struct DerivArgs {
     Fp *others, *tot, *totinv;
     size_t slots_pre;
     int n_blobs;
+    uint32_t *err; // error words, one per blob
 };
 
-__device__ __forceinline__ void deriv_pair(const DerivArgs &a, uint32_t p, const G1A *&pa, const G1A *&pb,
-                                           bool &neg_b) {
+__device__ __forceinline__ void deriv_pair(const DerivArgs &a, uint32_t p, PointRef &pa, PointRef &pb) {
     const uint32_t b = p / a.points, m = p - b * a.points;
     const DerivType ty = a.types[a.type_of[m]];
     const uint32_t n = a.parts.size[ty.part], off = a.parts.off[ty.part];
     const uint32_t x = m - ty.base;
     const bool wrap = x < ty.delta;
     const uint32_t xb = wrap ? x + n - ty.delta : x - ty.delta;
-    pa = &a.ladder_aff[((size_t)b * kCells + off + x) * kDigits + ty.row_a];
-    pb = &a.ladder_aff[((size_t)b * kCells + off + xb) * kDigits + ty.row_b];
-    neg_b = (ty.neg != 0) != (wrap && a.parts.nega[ty.part]);
+    pa = PointRef{&a.ladder_aff[((size_t)b * kCells + off + x) * kDigits + ty.row_a], false};
+    pb = PointRef{&a.ladder_aff[((size_t)b * kCells + off + xb) * kDigits + ty.row_b],
+                  (ty.neg != 0) != (wrap && a.parts.nega[ty.part])};
 }
 
-__device__ __forceinline__ void deriv_pass1_body(const DerivArgs &a, uint32_t gl, uint32_t NL) {
+template <class G>
+__device__ __forceinline__ void deriv_pass1_body(G &g, const DerivArgs &a, uint32_t gl, uint32_t NL) {
     const uint32_t wg = gl >> 5;
     const uint32_t P = (uint32_t)a.n_blobs * a.points;
     uint32_t *pre = a.pre + (size_t)wg * a.slots_pre * 384;
     Fp acc = fp_one();
-    int s = 0;
-    for (uint32_t p = gl; p < P; p += NL, s++) {
-        const G1A *pa, *pb;
-        bool nb;
-        deriv_pair(a, p, pa, pb, nb);
-        wb_store_pre(pre, s, acc);
-        acc = fp_mul(acc, pair_denominator_x(ld_vec(&pa->x), ld_vec(&pb->x), [&] { return ld_vec(pa); },
-                                             [&] {
-                                                 G1A y = ld_vec(pb);
-                                                 if (nb) y.y = fp_neg(y.y);
-                                                 return y;
-                                             }));
+    const int S = group_steps(P, gl, NL);
+    uint32_t p = gl;
+    for (int s = 0; s < S; s++, p += NL) {
+        PointRef x{nullptr, false}, y = x;
+        if (p < P) deriv_pair(a, p, x, y);
+        pass1_pair(g, acc, p < P, pre, s, x, y);
     }
-    flat_pass1_products(acc, a.others, a.tot, gl, wg);
+    flat_pass1_products(g, acc, a.others, a.tot, gl, wg);
 }
 __global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSM) k_deriv_pass1(DerivArgs a) {
-    deriv_pass1_body(a, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    __shared__ __align__(128) uint8_t tm_area[kTmSmem];
+    Tm g = tm_begin(tm_area);
+    deriv_pass1_body(g, a, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    tm_end(tm_area, a.err, (uint32_t)a.n_blobs);
 }
 
-__device__ __forceinline__ void deriv_pass2_body(const DerivArgs &a, uint32_t gl, uint32_t NL) {
+template <class G>
+__device__ __forceinline__ void deriv_pass2_body(G &g, const DerivArgs &a, uint32_t gl, uint32_t NL) {
     const uint32_t wg = gl >> 5;
     const uint32_t P = (uint32_t)a.n_blobs * a.points;
     const uint32_t *pre = a.pre + (size_t)wg * a.slots_pre * 384;
-    Fp inv = fp_mul(ld_vec(&a.totinv[wg]), ld_vec(&a.others[gl]));
-    const int S = P > gl ? (int)((P - gl + NL - 1) / NL) : 0;
-    for (int t = S - 1; t >= 0; t--) {
+    Fp inv = tm_mul<false>(g, ld_vec(&a.totinv[wg]), ld_vec(&a.others[gl]));
+    for (int t = group_steps(P, gl, NL) - 1; t >= 0; t--) {
         const uint32_t p = gl + (uint32_t)t * NL;
-        const G1A *pa, *pb;
-        bool nb;
-        deriv_pair(a, p, pa, pb, nb);
-        const G1A x = ld_vec(pa);
-        G1A y = ld_vec(pb);
-        if (nb) y.y = fp_neg(y.y);
-        const int kind = pair_kind(x, y);
-        const Fp den = pair_denominator(x, y, kind);
-        const Fp inv_den = fp_mul(inv, wb_load_pre(pre, t));
-        inv = fp_mul(inv, den);
-        st_vec(&a.out[p], pair_result(x, y, kind, inv_den));
+        PointRef x{nullptr, false}, y = x;
+        if (p < P) deriv_pair(a, p, x, y);
+        pass2_pair(g, inv, p < P, pre, t, x, y, &a.out[p]);
     }
 }
 __global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSM) k_deriv_pass2(DerivArgs a) {
-    deriv_pass2_body(a, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    __shared__ __align__(128) uint8_t tm_area[kTmSmem];
+    Tm g = tm_begin(tm_area);
+    deriv_pass2_body(g, a, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    tm_end(tm_area, a.err, (uint32_t)a.n_blobs);
 }
 
 // the shared pair sums into w.deriv_buf; returns the launches made (0 without any)
@@ -1640,6 +1682,7 @@ DerivArgs deriv_args(const DeviceTables &t, const ProofWork &w, int n) {
     a.totinv = w.flat_totinv;
     a.slots_pre = w.flat_slots;
     a.n_blobs = n;
+    a.err = w.err;
     return a;
 }
 
@@ -1670,48 +1713,54 @@ FlatBArgs flatb_args(const DeviceTables &t, const ProofWork &w, int n) {
     a.totinv = w.flat_totinv;
     a.slots = w.flat_slots;
     a.n_blobs = n;
+    a.err = w.err;
     return a;
 }
 
-VKZG_COOP_FN void coop_deriv_pass1(DerivArgs a, uint32_t gl, uint32_t NL) { deriv_pass1_body(a, gl, NL); }
-VKZG_COOP_FN void coop_deriv_pass2(DerivArgs a, uint32_t gl, uint32_t NL) { deriv_pass2_body(a, gl, NL); }
+VKZG_COOP_FN void coop_deriv_pass1(ScalarMul &t, DerivArgs a, uint32_t gl, uint32_t NL) { deriv_pass1_body(t, a, gl, NL); }
+VKZG_COOP_FN void coop_deriv_pass2(ScalarMul &t, DerivArgs a, uint32_t gl, uint32_t NL) { deriv_pass2_body(t, a, gl, NL); }
 template <bool FIRST>
-VKZG_COOP_FN void coop_flatb_pass1(FlatBArgs a, RoundIO io, int r, uint4 *smem, uint32_t gl, uint32_t NL) {
-    flatb_pass1_body<FIRST>(a, io, r, smem, gl, NL);
+VKZG_COOP_FN void coop_flatb_pass1(ScalarMul &t, FlatBArgs a, RoundIO io, int r, uint4 *smem, uint32_t gl, uint32_t NL) {
+    flatb_pass1_body<FIRST>(t, a, io, r, smem, gl, NL);
 }
 template <bool FIRST>
-VKZG_COOP_FN void coop_flatb_pass2(FlatBArgs a, RoundIO io, int r, uint4 *smem, uint32_t gl, uint32_t NL) {
-    flatb_pass2_body<FIRST>(a, io, r, smem, gl, NL);
+VKZG_COOP_FN void coop_flatb_pass2(ScalarMul &t, FlatBArgs a, RoundIO io, int r, uint4 *smem, uint32_t gl, uint32_t NL) {
+    flatb_pass2_body<FIRST>(t, a, io, r, smem, gl, NL);
 }
 
 // Cooperative form of the shared pair sums and phase B's rounds: one launch,
 // grid barriers between the passes (the arguments stay in the kernel's
 // parameters; only the round's lists change).
-__global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSM) k_coop_phase_b(DerivArgs da, int has_deriv, FlatBArgs fa,
-                                                                  G1A *buf0, G1A *buf1, int rounds, GridSync g) {
-    extern __shared__ uint4 dyn_smem[];
+__device__ __forceinline__ void coop_phase_b(ScalarMul &t, DerivArgs da, int has_deriv, FlatBArgs fa, G1A *buf0, G1A *buf1,
+                                             int rounds, GridSync g, uint4 *dyn_smem) {
     const uint32_t gl = blockIdx.x * blockDim.x + threadIdx.x, NL = gridDim.x * blockDim.x;
     if (has_deriv) {
-        coop_deriv_pass1(da, gl, NL);
+        coop_deriv_pass1(t, da, gl, NL);
         if (!grid_sync(g)) return;
         coop_invert(da.tot, da.totinv, NL >> 5, gl, NL);
         if (!grid_sync(g)) return;
-        coop_deriv_pass2(da, gl, NL);
+        coop_deriv_pass2(t, da, gl, NL);
         if (!grid_sync(g)) return;
     }
     RoundIO io{nullptr, buf0};
     for (int r = 0; r < rounds; r++) {
-        if (r == 0) coop_flatb_pass1<true>(fa, io, r, dyn_smem, gl, NL);
-        else coop_flatb_pass1<false>(fa, io, r, dyn_smem, gl, NL);
+        if (r == 0) coop_flatb_pass1<true>(t, fa, io, r, dyn_smem, gl, NL);
+        else coop_flatb_pass1<false>(t, fa, io, r, dyn_smem, gl, NL);
         if (!grid_sync(g)) return;
         coop_invert(fa.tot, fa.totinv, NL >> 5, gl, NL);
         if (!grid_sync(g)) return;
-        if (r == 0) coop_flatb_pass2<true>(fa, io, r, dyn_smem, gl, NL);
-        else coop_flatb_pass2<false>(fa, io, r, dyn_smem, gl, NL);
+        if (r == 0) coop_flatb_pass2<true>(t, fa, io, r, dyn_smem, gl, NL);
+        else coop_flatb_pass2<false>(t, fa, io, r, dyn_smem, gl, NL);
         io.src = io.dst;
         io.dst = io.dst == buf0 ? buf1 : buf0;
         if (r + 1 < rounds && !grid_sync(g)) return;
     }
+}
+__global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSM) k_coop_phase_b(DerivArgs da, int has_deriv, FlatBArgs fa,
+                                                                  G1A *buf0, G1A *buf1, int rounds, GridSync g) {
+    extern __shared__ uint4 dyn_smem[];
+    ScalarMul t;
+    coop_phase_b(t, da, has_deriv, fa, buf0, buf1, rounds, g, dyn_smem);
 }
 
 int launch_phase_b_coop(const DeviceTables &t, const ProofWork &w, int n, cudaStream_t s) {
@@ -2044,6 +2093,7 @@ struct FlatRArgs {
     Fp *others, *tot, *totinv;
     size_t slots_pre;
     int n_out;
+    uint32_t *err; // error words, one per blob
 };
 
 __device__ __forceinline__ G1A *red_slot(const FlatRArgs &a, uint32_t o, int s) {
@@ -2072,50 +2122,64 @@ __device__ void red_stage(RedRound &rr, int r) {
     __syncthreads();
 }
 
-__device__ __forceinline__ void flatr_pass1_body(const FlatRArgs &a, int r, RedRound &rr, uint32_t gl, uint32_t NL) {
+template <class G>
+__device__ __forceinline__ void flatr_pass1_body(G &g, const FlatRArgs &a, int r, RedRound &rr, uint32_t gl,
+                                                 uint32_t NL) {
     red_stage(rr, r);
     const uint32_t wg = gl >> 5;
     const uint32_t nops = (uint32_t)rr.nops;
     const uint32_t P = (uint32_t)a.n_out * nops;
     uint32_t *pre = a.pre + (size_t)wg * a.slots_pre * 384;
     Fp acc = fp_one();
-    int s = 0;
-    for (uint32_t p = gl; p < P; p += NL, s++) {
-        const uint32_t o = p / nops, q = p - o * nops;
-        const G1A *pa = red_slot(a, o, rr.a[q]), *pb = red_slot(a, o, rr.b[q]);
-        wb_store_pre(pre, s, acc);
-        acc = fp_mul(acc, pair_denominator_x(ld_vec(&pa->x), ld_vec(&pb->x), [&] { return ld_vec(pa); },
-                                             [&] { return ld_vec(pb); }));
+    const int S = group_steps(P, gl, NL);
+    uint32_t p = gl;
+    for (int s = 0; s < S; s++, p += NL) {
+        PointRef x{nullptr, false}, y = x;
+        if (p < P) {
+            const uint32_t o = p / nops, q = p - o * nops;
+            x.p = red_slot(a, o, rr.a[q]);
+            y.p = red_slot(a, o, rr.b[q]);
+        }
+        pass1_pair(g, acc, p < P, pre, s, x, y);
     }
-    flat_pass1_products(acc, a.others, a.tot, gl, wg);
+    flat_pass1_products(g, acc, a.others, a.tot, gl, wg);
 }
 __global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSM) k_flatr_pass1(FlatRArgs a, int r) {
     __shared__ RedRound rr;
-    flatr_pass1_body(a, r, rr, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    __shared__ __align__(128) uint8_t tm_area[kTmSmem];
+    Tm g = tm_begin(tm_area);
+    flatr_pass1_body(g, a, r, rr, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    tm_end(tm_area, a.err, (uint32_t)a.n_out / kCells);
 }
 
-__device__ __forceinline__ void flatr_pass2_body(const FlatRArgs &a, int r, RedRound &rr, uint32_t gl, uint32_t NL) {
+template <class G>
+__device__ __forceinline__ void flatr_pass2_body(G &g, const FlatRArgs &a, int r, RedRound &rr, uint32_t gl,
+                                                 uint32_t NL) {
     red_stage(rr, r);
     const uint32_t wg = gl >> 5;
     const uint32_t nops = (uint32_t)rr.nops;
     const uint32_t P = (uint32_t)a.n_out * nops;
     const uint32_t *pre = a.pre + (size_t)wg * a.slots_pre * 384;
-    Fp inv = fp_mul(ld_vec(&a.totinv[wg]), ld_vec(&a.others[gl]));
-    const int S = P > gl ? (int)((P - gl + NL - 1) / NL) : 0;
-    for (int t = S - 1; t >= 0; t--) {
+    Fp inv = tm_mul<false>(g, ld_vec(&a.totinv[wg]), ld_vec(&a.others[gl]));
+    for (int t = group_steps(P, gl, NL) - 1; t >= 0; t--) {
         const uint32_t p = gl + (uint32_t)t * NL;
-        const uint32_t o = p / nops, q = p - o * nops;
-        const G1A x = ld_vec(red_slot(a, o, rr.a[q])), y = ld_vec(red_slot(a, o, rr.b[q]));
-        const int kind = pair_kind(x, y);
-        const Fp den = pair_denominator(x, y, kind);
-        const Fp inv_den = fp_mul(inv, wb_load_pre(pre, t));
-        inv = fp_mul(inv, den);
-        st_vec(red_slot(a, o, rr.d[q]), pair_result(x, y, kind, inv_den));
+        PointRef x{nullptr, false}, y = x;
+        G1A *d = nullptr;
+        if (p < P) {
+            const uint32_t o = p / nops, q = p - o * nops;
+            x.p = red_slot(a, o, rr.a[q]);
+            y.p = red_slot(a, o, rr.b[q]);
+            d = red_slot(a, o, rr.d[q]);
+        }
+        pass2_pair(g, inv, p < P, pre, t, x, y, d);
     }
 }
 __global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSM) k_flatr_pass2(FlatRArgs a, int r) {
     __shared__ RedRound rr;
-    flatr_pass2_body(a, r, rr, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    __shared__ __align__(128) uint8_t tm_area[kTmSmem];
+    Tm g = tm_begin(tm_area);
+    flatr_pass2_body(g, a, r, rr, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    tm_end(tm_area, a.err, (uint32_t)a.n_out / kCells);
 }
 
 // H = sum_b 2^b T_b (Horner over the 7 bit sums), then + S: the reduction's result.
@@ -2140,26 +2204,30 @@ __global__ void __launch_bounds__(kCells) k_finish_horner(FlatRArgs a, uint8_t *
     finish_blob(outp, tree, proofs, b, t, levels);
 }
 
-VKZG_COOP_FN void coop_flatr_pass1(FlatRArgs a, int r, RedRound &rr, uint32_t gl, uint32_t NL) {
-    flatr_pass1_body(a, r, rr, gl, NL);
+VKZG_COOP_FN void coop_flatr_pass1(ScalarMul &t, FlatRArgs a, int r, RedRound &rr, uint32_t gl, uint32_t NL) {
+    flatr_pass1_body(t, a, r, rr, gl, NL);
 }
-VKZG_COOP_FN void coop_flatr_pass2(FlatRArgs a, int r, RedRound &rr, uint32_t gl, uint32_t NL) {
-    flatr_pass2_body(a, r, rr, gl, NL);
+VKZG_COOP_FN void coop_flatr_pass2(ScalarMul &t, FlatRArgs a, int r, RedRound &rr, uint32_t gl, uint32_t NL) {
+    flatr_pass2_body(t, a, r, rr, gl, NL);
 }
 
 // Cooperative form of the reduction's rounds (the Horner step stays its own
 // launch: one output per thread, a different register budget).
-__global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSM) k_coop_reduce(FlatRArgs a, int rounds, GridSync g) {
-    __shared__ RedRound rr;
+__device__ __forceinline__ void coop_reduce(ScalarMul &t, FlatRArgs a, int rounds, GridSync g, RedRound &rr) {
     const uint32_t gl = blockIdx.x * blockDim.x + threadIdx.x, NL = gridDim.x * blockDim.x;
     for (int r = 0; r < rounds; r++) {
-        coop_flatr_pass1(a, r, rr, gl, NL);
+        coop_flatr_pass1(t, a, r, rr, gl, NL);
         if (!grid_sync(g)) return;
         coop_invert(a.tot, a.totinv, NL >> 5, gl, NL);
         if (!grid_sync(g)) return;
-        coop_flatr_pass2(a, r, rr, gl, NL);
+        coop_flatr_pass2(t, a, r, rr, gl, NL);
         if (r + 1 < rounds && !grid_sync(g)) return;
     }
+}
+__global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSM) k_coop_reduce(FlatRArgs a, int rounds, GridSync g) {
+    __shared__ RedRound rr;
+    ScalarMul t;
+    coop_reduce(t, a, rounds, g, rr);
 }
 
 // proofs non-null: the Horner step runs inside stage 9 (k_finish_horner), which
@@ -2181,6 +2249,7 @@ int launch_reduce_flat(const ProofWork &w, const G1A *buckets, G1J *out, int n_o
     a.totinv = w.flat_totinv;
     a.slots_pre = w.flat_slots;
     a.n_out = n_out;
+    a.err = w.err;
     const int blocks = w.flat_blocks, warps = blocks * kFlatThreads / 32;
     int launched = 1;
     if (w.coop) {
@@ -2209,66 +2278,88 @@ struct NormArgs {
     Fp *others, *tot, *totinv;
     size_t slots_pre;
     uint32_t n;
+    uint32_t *err; // error words, one per blob
+    uint32_t n_err;
 };
 
-__device__ __forceinline__ void norm_pass1_body(const NormArgs &a, uint32_t gl, uint32_t NL) {
+template <class G>
+__device__ __forceinline__ void norm_pass1_body(G &g, const NormArgs &a, uint32_t gl, uint32_t NL) {
     const uint32_t wg = gl >> 5;
     uint32_t *pre = a.pre + (size_t)wg * a.slots_pre * 384;
     Fp acc = fp_one();
-    int s = 0;
-    for (uint32_t p = gl; p < a.n; p += NL, s++) {
-        const Fp z = ld_vec(&a.in[p].z);
-        wb_store_pre(pre, s, acc);
-        acc = fp_mul(acc, fp_is_zero(z) ? fp_one() : z);
+    const int S = group_steps(a.n, gl, NL);
+    uint32_t p = gl;
+    for (int s = 0; s < S; s++, p += NL) {
+        Fp z = fp_one();
+        if (p < a.n) {
+            wb_store_pre(pre, s, acc);
+            z = ld_vec(&a.in[p].z);
+            if (fp_is_zero(z)) z = fp_one();
+        }
+        acc = tm_mul<false>(g, acc, z);
     }
-    flat_pass1_products(acc, a.others, a.tot, gl, wg);
+    flat_pass1_products(g, acc, a.others, a.tot, gl, wg);
 }
 __global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSM) k_norm_pass1(NormArgs a) {
-    norm_pass1_body(a, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    __shared__ __align__(128) uint8_t tm_area[kTmSmem];
+    Tm g = tm_begin(tm_area);
+    norm_pass1_body(g, a, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    tm_end(tm_area, a.err, a.n_err);
 }
 
-__device__ __forceinline__ void norm_pass2_body(const NormArgs &a, uint32_t gl, uint32_t NL) {
+template <class G>
+__device__ __forceinline__ void norm_pass2_body(G &g, const NormArgs &a, uint32_t gl, uint32_t NL) {
     const uint32_t wg = gl >> 5;
     const uint32_t *pre = a.pre + (size_t)wg * a.slots_pre * 384;
-    Fp inv = fp_mul(ld_vec(&a.totinv[wg]), ld_vec(&a.others[gl]));
-    const int S = a.n > gl ? (int)((a.n - gl + NL - 1) / NL) : 0;
-    for (int t = S - 1; t >= 0; t--) {
+    Fp inv = tm_mul<false>(g, ld_vec(&a.totinv[wg]), ld_vec(&a.others[gl]));
+    for (int t = group_steps(a.n, gl, NL) - 1; t >= 0; t--) {
         const uint32_t p = gl + (uint32_t)t * NL;
-        const G1J q = ld_vec(&a.in[p]);
-        const bool inf = fp_is_zero(q.z);
-        const Fp zi = fp_mul(inv, wb_load_pre(pre, t));
-        inv = fp_mul(inv, inf ? fp_one() : q.z);
-        G1A r;
-        if (inf) {
-            r.x = fp_zero();
-            r.y = fp_zero();
-        } else {
-            const Fp z2 = fp_sqr(zi);
-            r.x = fp_mul(q.x, z2);
-            r.y = fp_mul(q.y, fp_mul(z2, zi));
+        const bool active = p < a.n;
+        Fp zi = fp_one(), z = fp_one();
+        bool inf = false;
+        if (active) {
+            zi = wb_load_pre(pre, t);
+            z = ld_vec(&a.in[p].z);
+            inf = fp_is_zero(z);
+            if (inf) z = fp_one();
         }
+        zi = tm_mul<false>(g, inv, zi);
+        inv = tm_mul<false>(g, inv, z);
+        // infinity: X = Y = 0 below gives (0, 0)
+        const Fp z2 = tm_sqr<false>(g, zi);
+        G1A r;
+        r.x = tm_mul<true>(g, active && !inf ? ld_vec(&a.in[p].x) : fp_zero(), z2);
+        r.y = tm_mul<true>(g, active && !inf ? ld_vec(&a.in[p].y) : fp_zero(), tm_mul<false>(g, z2, zi));
         // in: [row][16] ladder; out: [row][32], slot 16 + d = phi(slot d)
-        const size_t dst = (size_t)(p / kLadderDigits) * kDigits + p % kLadderDigits;
-        st_vec(&a.out[dst], r);
-        st_vec(&a.out[dst + kLadderDigits], g1_phi(r));
+        G1A *dst = &a.out[(size_t)(p / kLadderDigits) * kDigits + p % kLadderDigits];
+        if (active) st_vec(dst, r);
+        r.x = tm_mul<true>(g, r.x, g1_beta());
+        if (active) st_vec(dst + kLadderDigits, r);
     }
 }
 __global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSM) k_norm_pass2(NormArgs a) {
-    norm_pass2_body(a, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    __shared__ __align__(128) uint8_t tm_area[kTmSmem];
+    Tm g = tm_begin(tm_area);
+    norm_pass2_body(g, a, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    tm_end(tm_area, a.err, a.n_err);
 }
 
 // the ladder to affine form with its phi images, into w.ladder_aff; returns the launches made
-VKZG_COOP_FN void coop_norm_pass1(NormArgs a, uint32_t gl, uint32_t NL) { norm_pass1_body(a, gl, NL); }
-VKZG_COOP_FN void coop_norm_pass2(NormArgs a, uint32_t gl, uint32_t NL) { norm_pass2_body(a, gl, NL); }
+VKZG_COOP_FN void coop_norm_pass1(ScalarMul &t, NormArgs a, uint32_t gl, uint32_t NL) { norm_pass1_body(t, a, gl, NL); }
+VKZG_COOP_FN void coop_norm_pass2(ScalarMul &t, NormArgs a, uint32_t gl, uint32_t NL) { norm_pass2_body(t, a, gl, NL); }
 
 // Cooperative form of the ladder's normalisation round.
-__global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSM) k_coop_norm(NormArgs a, GridSync g) {
+__device__ __forceinline__ void coop_norm(ScalarMul &t, NormArgs a, GridSync g) {
     const uint32_t gl = blockIdx.x * blockDim.x + threadIdx.x, NL = gridDim.x * blockDim.x;
-    coop_norm_pass1(a, gl, NL);
+    coop_norm_pass1(t, a, gl, NL);
     if (!grid_sync(g)) return;
     coop_invert(a.tot, a.totinv, NL >> 5, gl, NL);
     if (!grid_sync(g)) return;
-    coop_norm_pass2(a, gl, NL);
+    coop_norm_pass2(t, a, gl, NL);
+}
+__global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSM) k_coop_norm(NormArgs a, GridSync g) {
+    ScalarMul t;
+    coop_norm(t, a, g);
 }
 
 int launch_normalize_flat(const ProofWork &w, int n, cudaStream_t s) {
@@ -2282,6 +2373,8 @@ int launch_normalize_flat(const ProofWork &w, int n, cudaStream_t s) {
     na.totinv = w.flat_totinv;
     na.slots_pre = w.flat_slots;
     na.n = (uint32_t)(n * kCells * kLadderDigits);
+    na.err = w.err;
+    na.n_err = (uint32_t)n;
     if (w.coop) {
         launch_coop(k_coop_norm, blocks, 0, s, na, make_sync(w, n));
         return 1;
@@ -2448,8 +2541,6 @@ cudaError_t configure_proof_kernels() {
     e = cudaFuncSetAttribute(k_flat_pass1<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStage1Bytes);
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(k_flat_pass2<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStage2Bytes);
-    if (e != cudaSuccess) return e;
-    e = configure_list_rounds();
     if (e != cudaSuccess) return e;
     return cudaFuncSetAttribute(k_phase_b_affine, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPhaseBSmem);
 }
