@@ -624,8 +624,9 @@ __device__ __forceinline__ void flat_pass1_products(G &g, const Fp &acc, Fp *oth
 #pragma unroll 1
     for (int d = 2; d < 32; d <<= 1) {
         const Fp partner = fp_shfl_xor(group, d);
-        rest = tm_mul<false>(g, rest, partner);
-        group = tm_mul<true>(g, group, partner);
+        tm_push_first(g, rest, partner);
+        rest = tm_push<false>(g, group, partner);
+        group = tm_pop<true>(g);
     }
     st_vec(&others[gl], rest);
     if (lane == 0) st_vec(&tot[wg], group);
@@ -656,48 +657,111 @@ __device__ __forceinline__ void pass1_pair(G &g, Fp &acc, bool active, uint32_t 
     acc = tm_mul<false>(g, acc, den);
 }
 
-// Pass 2 of one pair: its inverse denominator out of the running inverse, and the
-// sum to out.  The points are read again where they are needed (they are in
-// shared memory or in L1 by then) instead of being held across the products.
-template <class G, class A, class B>
-__device__ __forceinline__ void pass2_pair(G &g, Fp &inv, bool active, const uint32_t *pre, int t, A a, B b,
-                                           G1A *out) {
-    Fp den = fp_one(), num = fp_one(), lam = fp_one();
+// brings slot s's prefix products nearer: 12 lines of 128 bytes, one lane each
+__device__ __forceinline__ void wb_prefetch_pre(const uint32_t *pre, int s) {
+    const int lane = threadIdx.x & 31;
+    if (lane < 12) asm volatile("prefetch.global.L1 [%0];" ::"l"(pre + (size_t)(s * 12 + lane) * 32));
+}
+
+// A pair's denominator from the x coordinates, with its kind (pair_kind).
+template <class A, class B>
+__device__ __forceinline__ Fp pass2_denominator(const A &a, const B &b, int &kind) {
+    const Fp ax = a.x(), bx = b.x();
+    kind = 0;
+    if (!fp_is_zero(ax) && !fp_is_zero(bx) && !fp_eq(ax, bx)) return fp_sub(bx, ax);
+    const G1A p = a.point(), q = b.point();
+    kind = pair_kind(p, q);
+    return pair_denominator(p, q, kind);
+}
+template <class A, class B>
+__device__ __forceinline__ Fp pass2_numerator(const A &a, const B &b, int kind) {
+    if (kind != 1) return fp_sub(b.y(), a.y());
+    const Fp xx = fp_sqr(a.x());
+    return fp_add(fp_dbl(xx), xx);
+}
+
+// Pass 2 of a lane's pairs, the last slot first: with the running inverse inv (of
+// the denominators of slots 0..t) and the prefix product pre_t,
+//   A_t = inv pre_t = 1 / den_t,   B_t = inv den_t, the next inv,
+//   L_t = num_t A_t,   x3 = L_t^2 - ax - bx,   y3 = L_t (ax - x3) - ay.
+// The products of pair t alternate with A and B of pair t - 1, so that none needs
+// the one pushed just before it and every trip to the tensor core runs behind the
+// next product's multiplications.  The points are read again where they are
+// needed (from shared memory or L1) instead of being held across the products.
+// Per warp pair of the second round at 64 blobs the sequential form took 39 % of
+// the issue slots, waiting for the tensor core.
+// src.pair(t, active): slot t's points and destination, asked for once, t
+// descending from S - 1; src.done(t): slot t's points are no longer needed.  own:
+// the lane's pairs, S or S - 1.
+template <class G, class Src>
+__device__ __forceinline__ void pass2_pairs(G &g, Fp inv, int S, int own, const uint32_t *pre, Src &src) {
+    if (S <= 0) return;
+    auto cur = src.pair(S - 1, S - 1 < own);
     int kind = 0;
-    if (active) {
-        lam = wb_load_pre(pre, t);
-        const G1A p = a.point(), q = b.point();
-        kind = pair_kind(p, q);
-        den = pair_denominator(p, q, kind);
-        if (kind == 1) {
-            const Fp xx = fp_sqr(p.x);
-            num = fp_add(fp_dbl(xx), xx);
+    Fp A, L;
+    {
+        const bool active = S - 1 < own;
+        Fp v = fp_one();
+        if (active) v = wb_load_pre(pre, S - 1);
+        tm_push_first(g, inv, v);
+        v = fp_one();
+        if (active) v = pass2_denominator(cur.a, cur.b, kind);
+        A = tm_push<false>(g, inv, v);
+        v = fp_one();
+        if (active) v = pass2_numerator(cur.a, cur.b, kind);
+        inv = tm_push<false>(g, v, A);
+    }
+#pragma unroll 1
+    for (int t = S - 1;; t--) {
+        const bool active = t < own;
+        auto nxt = cur;
+        int kind_n = 0;
+        Fp d;
+        G1A r;
+        if (t > 0) { // slots below S - 1 are all the lane's own
+            nxt = src.pair(t - 1, true);
+            const Fp v = wb_load_pre(pre, t - 1);
+            if (t > 1) wb_prefetch_pre(pre, t - 2);
+            L = tm_push<false>(g, inv, v);
+            A = tm_push_sqr<false>(g, L);
+            r.x = tm_push<true>(g, inv, pass2_denominator(nxt.a, nxt.b, kind_n));
         } else {
-            num = fp_sub(q.y, p.y);
+            L = tm_pop<false>(g);
+            r.x = tm_sqr<true>(g, L);
         }
-    }
-    lam = tm_mul<false>(g, inv, lam);
-    inv = tm_mul<false>(g, inv, den);
-    lam = tm_mul<false>(g, num, lam);
-    G1A r;
-    r.x = tm_sqr<true>(g, lam);
-    Fp d = fp_zero();
-    if (active) {
-        const Fp ax = a.x();
-        r.x = fp_sub(fp_sub(r.x, ax), b.x());
-        d = fp_sub(ax, r.x);
-    }
-    r.y = tm_mul<true>(g, lam, d);
-    if (active) {
-        r.y = fp_sub(r.y, a.y());
-        if (kind >= 2) { // rare: infinity on a side, or a point and its negative
-            r = G1A{fp_zero(), fp_zero()};
-            if (kind == 2) r = a.point();
-            if (kind == 3) r = b.point();
+        d = fp_zero();
+        if (active) {
+            const Fp ax = cur.a.x();
+            r.x = fp_sub(fp_sub(r.x, ax), cur.b.x());
+            d = fp_sub(ax, r.x);
         }
-        st_vec(out, r);
+        if (t > 0) {
+            inv = tm_push<false>(g, L, d);
+            r.y = tm_push<true>(g, pass2_numerator(nxt.a, nxt.b, kind_n), A);
+        } else {
+            r.y = tm_mul<true>(g, L, d);
+        }
+        if (active) {
+            r.y = fp_sub(r.y, cur.a.y());
+            if (kind >= 2) { // rare: infinity on a side, or a point and its negative
+                r = G1A{fp_zero(), fp_zero()};
+                if (kind == 2) r = cur.a.point();
+                if (kind == 3) r = cur.b.point();
+            }
+            st_vec(cur.out, r);
+        }
+        if (t == 0) return;
+        src.done(t);
+        cur = nxt;
+        kind = kind_n;
     }
 }
+
+// a pair of points in memory and where their sum goes
+struct PairRefs {
+    PointRef a, b;
+    G1A *out;
+};
 
 // A round's input and output lists, apart from the phase's other arguments:
 // a cooperative launch changes them every round while the rest stays in the
@@ -947,91 +1011,99 @@ __device__ __forceinline__ void flat_odd_points(const FlatArgs &a, RoundIO io, u
         st_vec(&io.dst[(size_t)l * ((m + 1) >> 1) + (m >> 1)], flat_ref<FIRST>(a, io, l, m - 1, m).point());
 }
 
-// pass 2 with the two points of each pair staged one pair ahead from the digit table
-template <class G>
-__device__ __forceinline__ void flat_pass2_staged(G &g, const FlatArgs &a, RoundIO io, uint32_t m, uint32_t gl,
-                                                  uint32_t NL) {
-    extern __shared__ uint4 stage[];
-    uint4 *my = stage + threadIdx.x; // chunk c of buffer b: my[(b * kStageChunks + c) * kFlatThreads]
-    const uint32_t wg = gl >> 5;
-    const uint32_t h = m >> 1, m_next = (m + 1) >> 1;
-    const uint32_t P = (uint32_t)a.n_lists * h;
-    const uint32_t dq = NL / h, dr = NL % h;
-    const uint32_t *pre = a.pre + (size_t)wg * a.slots * 384;
-    auto issue = [&](int b, uint32_t o, uint32_t i, int &v0, int &v1) {
-        const int16_t *d = a.dig + (size_t)o * a.L + 2 * i;
-        v0 = d[0];
-        v1 = d[1];
-        if (v0) {
-            const uint4 *src = comb_entry(a, o, 2 * i, v0);
-            for (int c = 0; c < 6; c++) cp_async16(&my[(b * kStageChunks + c) * kFlatThreads], src + c);
-        }
-        if (v1) {
-            const uint4 *src = comb_entry(a, o, 2 * i + 1, v1);
-            for (int c = 0; c < 6; c++) cp_async16(&my[(b * kStageChunks + 6 + c) * kFlatThreads], src + c);
+// Pass 2's pairs of a tree round, their points staged in shared memory from the
+// digit table (FIRST) or from the round's lists two slots ahead of their use.
+template <bool FIRST>
+struct FlatPairs {
+    const FlatArgs &a;
+    RoundIO io;
+    uint32_t m, h, m_next, dq, dr;
+    uint4 *my;                     // chunk c of buffer b: my[(b * kStageChunks + c) * kFlatThreads]
+    uint32_t o, i;                 // the slot staged last
+    int staged;                    // its index
+    int v[2][2];                   // the buffers' digits
+    uint32_t at[2];                // and where their sums go
+    struct Pair {
+        StagedRef a, b;
+        G1A *out;
+    };
+    __device__ __forceinline__ void stage(int t) {
+        const int b = t & 1;
+        uint4 *w = my + b * kStageChunks * kFlatThreads;
+        int v0 = 1, v1 = 1;
+        if constexpr (FIRST) {
+            const int16_t *d = a.dig + (size_t)o * a.L + 2 * i;
+            v0 = d[0];
+            v1 = d[1];
+            if (v0) {
+                const uint4 *src = comb_entry(a, o, 2 * i, v0);
+                for (int c = 0; c < 6; c++) cp_async16(&w[c * kFlatThreads], src + c);
+            }
+            if (v1) {
+                const uint4 *src = comb_entry(a, o, 2 * i + 1, v1);
+                for (int c = 0; c < 6; c++) cp_async16(&w[(6 + c) * kFlatThreads], src + c);
+            }
+        } else { // the pair's two points, 192 contiguous bytes of the list
+            const uint4 *src = reinterpret_cast<const uint4 *>(&io.src[(size_t)o * m + 2 * i]);
+            for (int c = 0; c < kStageChunks; c++) cp_async16(&w[c * kFlatThreads], src + c);
         }
         cp_async_commit();
-    };
-    const int S = group_steps(P, gl, NL);
-    const int own = P > gl ? (int)((P - gl + NL - 1) / NL) : 0; // S or S - 1
-    uint32_t o = 0, i = 0;
-    int v0 = 0, v1 = 0;
-    if (own > 0) {
+        if (b) {
+            v[1][0] = v0;
+            v[1][1] = v1;
+            at[1] = o * m_next + i;
+        } else {
+            v[0][0] = v0;
+            v[0][1] = v1;
+            at[0] = o * m_next + i;
+        }
+        staged = t;
+    }
+    // stages the lane's last two slots
+    __device__ __forceinline__ void begin(uint32_t gl, uint32_t NL, int own) {
+        if (own <= 0) return;
         const uint32_t p_last = gl + (uint32_t)(own - 1) * NL;
         o = p_last / h;
         i = p_last % h;
-        issue((own - 1) & 1, o, i, v0, v1);
-    }
-    Fp inv = tm_mul<false>(g, ld_vec(&a.totinv[wg]), ld_vec(&a.others[gl]));
-    for (int t = S - 1; t >= 0; t--) {
-        const bool active = t < own;
-        uint32_t on = o, in = i;
-        int w0 = v0, w1 = v1;
-        if (active && t > 0) {
-            pair_step_down(on, in, h, dq, dr);
-            issue((t - 1) & 1, on, in, w0, w1);
-            cp_async_wait<1>();
-        } else if (active) {
-            cp_async_wait<0>();
+        stage(own - 1);
+        if (own > 1) {
+            pair_step_down(o, i, h, dq, dr);
+            stage(own - 2);
         }
-        const uint4 *w = my + (t & 1) * kStageChunks * kFlatThreads;
-        pass2_pair(g, inv, active, pre, t, StagedRef{w, v0}, StagedRef{w + 6 * kFlatThreads, v1},
-                   &io.dst[(size_t)o * m_next + i]);
-        o = on;
-        i = in;
-        v0 = w0;
-        v1 = w1;
     }
-    flat_odd_points<true>(a, io, m, gl, NL);
-}
+    __device__ __forceinline__ Pair pair(int t, bool active) {
+        if (active) {
+            if (staged < t) cp_async_wait<1>();
+            else cp_async_wait<0>();
+        }
+        const int b = t & 1;
+        const uint4 *w = my + b * kStageChunks * kFlatThreads;
+        return Pair{StagedRef{w, b ? v[1][0] : v[0][0]}, StagedRef{w + 6 * kFlatThreads, b ? v[1][1] : v[0][1]},
+                    &io.dst[b ? at[1] : at[0]]};
+    }
+    __device__ __forceinline__ void done(int t) {
+        // t is below own here except for a neutral first slot, after which both buffers are still in use
+        if (t >= 2 && staged == t - 1) {
+            pair_step_down(o, i, h, dq, dr);
+            stage(t - 2);
+        }
+    }
+};
 
 template <bool FIRST, class G>
 __device__ __forceinline__ void flat_pass2_body(G &g, const FlatArgs &a, RoundIO io, uint32_t m, uint32_t gl,
                                                 uint32_t NL) {
-    if constexpr (FIRST) {
-        flat_pass2_staged(g, a, io, m, gl, NL);
-        return;
-    }
+    extern __shared__ uint4 stage[];
     const uint32_t wg = gl >> 5;
-    const uint32_t h = m >> 1, m_next = (m + 1) >> 1;
+    const uint32_t h = m >> 1;
     const uint32_t P = (uint32_t)a.n_lists * h;
-    const uint32_t dq = NL / h, dr = NL % h;
-    const uint32_t *pre = a.pre + (size_t)wg * a.slots * 384;
-    Fp inv = tm_mul<false>(g, ld_vec(&a.totinv[wg]), ld_vec(&a.others[gl]));
     const int S = group_steps(P, gl, NL);
     const int own = P > gl ? (int)((P - gl + NL - 1) / NL) : 0; // S or S - 1
-    uint32_t o = 0, i = 0;
-    if (own > 0) {
-        const uint32_t p_last = gl + (uint32_t)(own - 1) * NL;
-        o = p_last / h;
-        i = p_last % h;
-    }
-    for (int t = S - 1; t >= 0; t--) {
-        pass2_pair(g, inv, t < own, pre, t, flat_ref<false>(a, io, o, 2 * i, m), flat_ref<false>(a, io, o, 2 * i + 1, m),
-                   &io.dst[(size_t)o * m_next + i]);
-        if (t < own && t > 0) pair_step_down(o, i, h, dq, dr);
-    }
-    flat_odd_points<false>(a, io, m, gl, NL);
+    FlatPairs<FIRST> src{a, io, m, h, (m + 1) >> 1, NL / h, NL % h, stage + threadIdx.x, 0, 0, 0, {{0, 0}, {0, 0}}, {0, 0}};
+    src.begin(gl, NL, own);
+    const Fp inv = tm_mul<false>(g, ld_vec(&a.totinv[wg]), ld_vec(&a.others[gl]));
+    pass2_pairs(g, inv, S, own, a.pre + (size_t)wg * a.slots * 384, src);
+    flat_odd_points<FIRST>(a, io, m, gl, NL);
 }
 
 template <bool FIRST>
@@ -1111,8 +1183,8 @@ const G1A *run_tree_rounds(FlatArgs a, const G1A *first_src, uint32_t *m_io, uin
         if (first) k_flat_pass1<FIRST><<<blocks, kFlatThreads, FIRST ? kStage1Bytes : 0, s>>>(a, m);
         else k_flat_pass1<false><<<blocks, kFlatThreads, 0, s>>>(a, m);
         launch_flat_invert(a.tot, a.totinv, warps, s);
-        if (first) k_flat_pass2<FIRST><<<blocks, kFlatThreads, FIRST ? kStage2Bytes : 0, s>>>(a, m);
-        else k_flat_pass2<false><<<blocks, kFlatThreads, 0, s>>>(a, m);
+        if (first) k_flat_pass2<FIRST><<<blocks, kFlatThreads, kStage2Bytes, s>>>(a, m);
+        else k_flat_pass2<false><<<blocks, kFlatThreads, kStage2Bytes, s>>>(a, m);
         *launched += 3;
         cur = bufs[out];
         out ^= 1;
@@ -1137,6 +1209,9 @@ int launch_tree_sums(const G1A *lists, int n_lists, uint32_t m, G1A *buf0, G1A *
     a.slots = slots;
     a.n_lists = n_lists;
     int launched = 0;
+    if (cudaFuncSetAttribute(k_flat_pass2<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStage2Bytes) !=
+        cudaSuccess)
+        return 0;
     const G1A *res = run_tree_rounds<false>(a, lists, &m, 1, buf0, buf1, blocks, s, &launched);
     cudaMemcpyAsync(sums, res, (size_t)n_lists * sizeof(G1A), cudaMemcpyDeviceToDevice, s);
     count_launches(launched);
@@ -1309,7 +1384,7 @@ int launch_phase_a_flat(const ProofWork &w, int n, cudaStream_t s) {
                     w.flat_buf[1], m0, (m0 + 1) >> 1, make_sync(w, n));
         launched++;
         if (((m0 + 1) >> 1) > kTreeTail) {
-            launch_coop(k_coop_tree<false>, w.flat_blocks, 0, s, a, (const G1A *)w.flat_buf[0], w.flat_buf[1],
+            launch_coop(k_coop_tree<false>, w.flat_blocks, kStage2Bytes, s, a, (const G1A *)w.flat_buf[0], w.flat_buf[1],
                         w.flat_buf[0], (m0 + 1) >> 1, kTreeTail, make_sync(w, n));
             launched++;
         }
@@ -1530,22 +1605,29 @@ __device__ __forceinline__ void flatb_pass2_body(G &g, const FlatBArgs &a, Round
     const uint32_t P = sr.pair_end[sr.n_parts - 1];
     const uint32_t *pre = a.pre + (size_t)wg * a.slots * 384;
     const bool last = r + 1 == a.plan->rounds;
-    Fp inv = tm_mul<false>(g, ld_vec(&a.totinv[wg]), ld_vec(&a.others[gl]));
-    for (int t = group_steps(P, gl, NL) - 1; t >= 0; t--) {
-        const uint32_t p = gl + (uint32_t)t * NL;
-        PointRef x{nullptr, false}, y = x;
-        G1A *d = nullptr;
-        if (p < P) {
+    const Fp inv = tm_mul<false>(g, ld_vec(&a.totinv[wg]), ld_vec(&a.others[gl]));
+    struct {
+        const FlatBArgs &a;
+        RoundIO io;
+        const FlatBRound &sr;
+        const uint32_t *items, *offs;
+        uint32_t gl, NL;
+        bool last;
+        __device__ __forceinline__ PairRefs pair(int t, bool active) const {
+            PairRefs r{{nullptr, false}, {nullptr, false}, nullptr};
+            if (!active) return r;
             uint32_t o, i;
             int q, k;
-            flatb_pair(sr, p, o, q, k, i);
-            x = flatb_ref<FIRST>(a, io, sr, items, offs, o, q, k, 2 * i);
-            y = flatb_ref<FIRST>(a, io, sr, items, offs, o, q, k, 2 * i + 1);
-            d = last ? &a.bucket_aff[(size_t)o * kBuckets + k]
-                     : &io.dst[(size_t)o * sr.stride_next + sr.base_next[q][k] + i];
+            flatb_pair(sr, gl + (uint32_t)t * NL, o, q, k, i);
+            r.a = flatb_ref<FIRST>(a, io, sr, items, offs, o, q, k, 2 * i);
+            r.b = flatb_ref<FIRST>(a, io, sr, items, offs, o, q, k, 2 * i + 1);
+            r.out = last ? &a.bucket_aff[(size_t)o * kBuckets + k]
+                         : &io.dst[(size_t)o * sr.stride_next + sr.base_next[q][k] + i];
+            return r;
         }
-        pass2_pair(g, inv, p < P, pre, t, x, y, d);
-    }
+        __device__ __forceinline__ void done(int) const {}
+    } src{a, io, sr, items, offs, gl, NL, last};
+    pass2_pairs(g, inv, group_steps(P, gl, NL), P > gl ? (int)((P - gl + NL - 1) / NL) : 0, pre, src);
     // odd last elements move up unchanged
     const FlatBPlan &pl = *a.plan;
     size_t odd_begin = 0;
@@ -1652,13 +1734,21 @@ __device__ __forceinline__ void deriv_pass2_body(G &g, const DerivArgs &a, uint3
     const uint32_t wg = gl >> 5;
     const uint32_t P = (uint32_t)a.n_blobs * a.points;
     const uint32_t *pre = a.pre + (size_t)wg * a.slots_pre * 384;
-    Fp inv = tm_mul<false>(g, ld_vec(&a.totinv[wg]), ld_vec(&a.others[gl]));
-    for (int t = group_steps(P, gl, NL) - 1; t >= 0; t--) {
-        const uint32_t p = gl + (uint32_t)t * NL;
-        PointRef x{nullptr, false}, y = x;
-        if (p < P) deriv_pair(a, p, x, y);
-        pass2_pair(g, inv, p < P, pre, t, x, y, &a.out[p]);
-    }
+    const Fp inv = tm_mul<false>(g, ld_vec(&a.totinv[wg]), ld_vec(&a.others[gl]));
+    struct {
+        const DerivArgs &a;
+        uint32_t gl, NL;
+        __device__ __forceinline__ PairRefs pair(int t, bool active) const {
+            PairRefs r{{nullptr, false}, {nullptr, false}, nullptr};
+            if (!active) return r;
+            const uint32_t p = gl + (uint32_t)t * NL;
+            deriv_pair(a, p, r.a, r.b);
+            r.out = &a.out[p];
+            return r;
+        }
+        __device__ __forceinline__ void done(int) const {}
+    } src{a, gl, NL};
+    pass2_pairs(g, inv, group_steps(P, gl, NL), P > gl ? (int)((P - gl + NL - 1) / NL) : 0, pre, src);
 }
 __global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSM) k_deriv_pass2(DerivArgs a) {
     __shared__ __align__(128) uint8_t tm_area[kTmSmem];
@@ -2160,19 +2250,23 @@ __device__ __forceinline__ void flatr_pass2_body(G &g, const FlatRArgs &a, int r
     const uint32_t nops = (uint32_t)rr.nops;
     const uint32_t P = (uint32_t)a.n_out * nops;
     const uint32_t *pre = a.pre + (size_t)wg * a.slots_pre * 384;
-    Fp inv = tm_mul<false>(g, ld_vec(&a.totinv[wg]), ld_vec(&a.others[gl]));
-    for (int t = group_steps(P, gl, NL) - 1; t >= 0; t--) {
-        const uint32_t p = gl + (uint32_t)t * NL;
-        PointRef x{nullptr, false}, y = x;
-        G1A *d = nullptr;
-        if (p < P) {
-            const uint32_t o = p / nops, q = p - o * nops;
-            x.p = red_slot(a, o, rr.a[q]);
-            y.p = red_slot(a, o, rr.b[q]);
-            d = red_slot(a, o, rr.d[q]);
+    const Fp inv = tm_mul<false>(g, ld_vec(&a.totinv[wg]), ld_vec(&a.others[gl]));
+    struct {
+        const FlatRArgs &a;
+        const RedRound &rr;
+        uint32_t gl, NL, nops;
+        __device__ __forceinline__ PairRefs pair(int t, bool active) const {
+            PairRefs r{{nullptr, false}, {nullptr, false}, nullptr};
+            if (!active) return r;
+            const uint32_t p = gl + (uint32_t)t * NL, o = p / nops, q = p - o * nops;
+            r.a.p = red_slot(a, o, rr.a[q]);
+            r.b.p = red_slot(a, o, rr.b[q]);
+            r.out = red_slot(a, o, rr.d[q]);
+            return r;
         }
-        pass2_pair(g, inv, p < P, pre, t, x, y, d);
-    }
+        __device__ __forceinline__ void done(int) const {}
+    } src{a, rr, gl, NL, nops};
+    pass2_pairs(g, inv, group_steps(P, gl, NL), P > gl ? (int)((P - gl + NL - 1) / NL) : 0, pre, src);
 }
 __global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSM) k_flatr_pass2(FlatRArgs a, int r) {
     __shared__ RedRound rr;
@@ -2522,11 +2616,14 @@ bool coop_supported(int blocks_per_sm) {
     if (cudaFuncSetAttribute(k_coop_tree<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStage2Bytes) !=
         cudaSuccess)
         return false;
+    if (cudaFuncSetAttribute(k_coop_tree<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStage2Bytes) !=
+        cudaSuccess)
+        return false;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_coop_tree<true>, kFlatThreads, kStage2Bytes);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_coop_norm, kFlatThreads, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, k_coop_phase_b, kFlatThreads, kFlatBSmem);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d, k_coop_reduce, kFlatThreads, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&e, k_coop_tree<false>, kFlatThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&e, k_coop_tree<false>, kFlatThreads, kStage2Bytes);
     return std::min(std::min(std::min(a, b), std::min(c, d)), e) >= blocks_per_sm;
 }
 
@@ -2541,6 +2638,8 @@ cudaError_t configure_proof_kernels() {
     e = cudaFuncSetAttribute(k_flat_pass1<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStage1Bytes);
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(k_flat_pass2<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStage2Bytes);
+    if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(k_flat_pass2<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStage2Bytes);
     if (e != cudaSuccess) return e;
     return cudaFuncSetAttribute(k_phase_b_affine, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPhaseBSmem);
 }

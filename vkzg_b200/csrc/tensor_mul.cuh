@@ -190,13 +190,20 @@ constexpr TmImage tm_image() {
 // ---- device side: groups of 128 threads (four warps, one row of the matrix
 // product each) share a block's copy of the constant matrix.
 constexpr int kTmGroup = 128;
-constexpr int kTmTmemCols = 128;   // TMEM columns of a group: its bytes from column 0, the sums from kTmSums
-constexpr int kTmSums = 64;
+// TMEM columns of a group: two areas for a product's bytes (one filled while the
+// tensor core reads the other), then the sums
+constexpr int kTmTmemCols = 128;
+constexpr int kTmBytes = kTmRowsPad / 4;
+constexpr int kTmSums = 2 * kTmBytes;
+static_assert(kTmSums + kTmCols <= kTmTmemCols, "the areas fit a group's columns");
 constexpr int kTmMatrixBytes = kTmRowsPad * kTmCols;
 // a block's shared memory: the matrix, then one mbarrier per group (at most
-// kTmMaxGroups), the TMEM address, and the flag that a wait gave up
-constexpr int kTmMaxGroups = 2; // tm_exchange names a barrier for each
-constexpr int kTmSmem = kTmMatrixBytes + 8 * kTmMaxGroups + 16;
+// kTmMaxGroups), the TMEM address, the flag that a wait gave up, and one count of
+// arrived warps per group
+constexpr int kTmMaxGroups = 2;
+constexpr int kTmCounts = kTmMatrixBytes + 8 * kTmMaxGroups + 8;
+constexpr int kTmSmem = kTmCounts + 4 * kTmMaxGroups;
+static_assert(kTmGroup == 128, "a count of four warps per product");
 // polls of a wait for the tensor core (each suspends up to kTmPollNs) before it gives up
 constexpr uint32_t kTmPolls = 20000, kTmPollNs = 2000;
 
@@ -204,8 +211,10 @@ __device__ const TmImage d_tm_image = tm_image();
 
 struct Tm {
     uint32_t t;  // the warp's TMEM address
-    uint32_t sm; // shared address of the block's area (128-byte aligned), bit 0: the mbarrier's phase
+    uint32_t sm; // shared address of the block's area (128-byte aligned); bit 0: the
+                 // mbarrier's phase, bit 1: the byte area of the next product
 };
+constexpr uint32_t kTmFlags = 3u;
 
 __device__ __forceinline__ uint32_t tm_smem(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -219,7 +228,7 @@ __device__ __forceinline__ Tm tm_begin(uint8_t *area) {
     uint32_t *word = reinterpret_cast<uint32_t *>(area + kTmMatrixBytes + 8 * kTmMaxGroups);
     if (threadIdx.x < kTmMaxGroups)
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars + 8 * threadIdx.x) : "memory");
-    if (threadIdx.x == 0) word[1] = 0;
+    if (threadIdx.x <= kTmMaxGroups) word[1 + threadIdx.x] = 0; // the flag, the counts
     if (threadIdx.x < 32) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tm_smem(word)),
                      "n"(kTmMaxGroups * kTmTmemCols)
@@ -260,35 +269,48 @@ __device__ __forceinline__ void tm_put(uint32_t t, const uint32_t *z) {
                  : "memory");
 }
 
-// The group's matrix product over the bytes put, and the sums of this thread's
-// row: columns joined in pairs (weight 2^(16 k); each below 144 * 255^2 * 257 < 2^32).
-// Called by whole groups.
-__device__ __forceinline__ void tm_exchange(uint32_t t, uint32_t sm_phase, uint32_t *w) {
-    const uint32_t sm = sm_phase & ~1u, phase = sm_phase & 1u, grp = threadIdx.x / kTmGroup;
-    const uint32_t bar = sm + kTmMatrixBytes + 8 * grp;
+// Starts the group's matrix product over the bytes put, once every warp of the
+// group has put its rows and read the sums of the product before: each warp
+// counts itself in and goes on, and the one that completes the count issues the
+// product.  (A barrier of the group in its place cost 1.4 of 9.2 cycles per
+// issued instruction in the second round's pass 2.)  Called by whole groups, as
+// is everything below.
+__device__ __forceinline__ void tm_start(uint32_t t, uint32_t ctl) {
+    const uint32_t sm = ctl & ~kTmFlags, grp = threadIdx.x / kTmGroup;
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    // barrier ids as constants: with an id in a register the kernel is given all
-    // 16, and one block per SM
-    if (grp == 0) asm volatile("bar.sync 1, %0;" ::"n"(kTmGroup) : "memory");
-    else asm volatile("bar.sync 2, %0;" ::"n"(kTmGroup) : "memory");
-    if ((threadIdx.x & (kTmGroup - 1)) == 0) {
+    __syncwarp();
+    uint32_t in = 0;
+    if ((threadIdx.x & 31) == 0)
+        asm volatile("atom.acq_rel.cta.shared.add.u32 %0, [%1], 1;"
+                     : "=r"(in)
+                     : "r"(sm + kTmCounts + 4 * grp)
+                     : "memory");
+    if ((threadIdx.x & 31) == 0 && (in & 3u) == 3u) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         // S32 sums, U8 x U8, both K-major, 128 x kTmCols x 32 a step
         constexpr uint32_t idesc = (2u << 4) | ((kTmCols / 8) << 17) | ((kTmGroup / 16) << 24);
         // no swizzle: core matrices kTmCols * 16 bytes apart along K, 128 along N
         const uint64_t desc = (uint64_t)(sm >> 4) | ((uint64_t)kTmCols << 16) | ((uint64_t)8 << 32) | (1ull << 46);
-        const uint32_t base = t & 0xffffu;
+        const uint32_t base = t & 0xffffu, bytes = base + (ctl & 2u) / 2 * kTmBytes;
 #pragma unroll
         for (int s = 0; s < kTmRowsPad / 32; s++)
             asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
                          "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}" ::"r"(base + kTmSums),
-                         "r"(base + 8 * s), "l"(desc + (uint64_t)(2 * kTmCols * s)), "r"(idesc), "r"(s)
+                         "r"(bytes + 8 * s), "l"(desc + (uint64_t)(2 * kTmCols * s)), "r"(idesc), "r"(s)
                          : "memory");
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                         sm + kTmMatrixBytes + 8 * grp)
                      : "memory");
     }
     __syncwarp();
+}
+
+// Waits for the matrix product started last and reads the sums of this thread's
+// row: columns joined in pairs (weight 2^(16 k); each below 144 * 255^2 * 257 < 2^32).
+__device__ __forceinline__ void tm_sums(uint32_t t, uint32_t ctl, uint32_t *w) {
+    const uint32_t sm = ctl & ~kTmFlags, phase = ctl & 1u, grp = threadIdx.x / kTmGroup;
+    const uint32_t bar = sm + kTmMatrixBytes + 8 * grp;
     uint32_t ok = 0, polls = 0;
     do {
         asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
@@ -325,72 +347,143 @@ __device__ __forceinline__ void tm_exchange(uint32_t t, uint32_t sm_phase, uint3
     for (int k = 0; k < kTmCols / 2; k++) w[k] = c[2 * k] + (c[2 * k + 1] << 8);
 }
 
-// CANON: the product in [0, p); else in [0, p + 2^365).  Operands below 2^382.
-template <bool CANON>
+// The product, in [0, p + 2^365) for operands below 2^382.
 __device__ __forceinline__ Fp tm_result(const uint32_t *w) {
-    Fp t;
-    tm_join(t.v, w);
-    if (!CANON) return t;
+    Fp r;
+    tm_join(r.v, w);
+    return r;
+}
+// a value below 2p in [0, p)
+__device__ __forceinline__ Fp tm_canonical(const Fp &a) {
     CARRY_DECL
+    Fp r;
     uint32_t s[12], borrow;
-    SUB_CC(s[0], t.v[0], fp_p(0));
+    SUB_CC(s[0], a.v[0], fp_p(0));
 #pragma unroll
-    for (int i = 1; i < 12; i++) SUBC_CC(s[i], t.v[i], fp_p(i));
+    for (int i = 1; i < 12; i++) SUBC_CC(s[i], a.v[i], fp_p(i));
     SUBC(borrow, 0u, 0u);
 #pragma unroll
-    for (int i = 0; i < 12; i++) t.v[i] = borrow ? t.v[i] : s[i];
-    return t;
+    for (int i = 0; i < 12; i++) r.v[i] = borrow ? a.v[i] : s[i];
+    return r;
 }
 template <bool CANON>
-__device__ __noinline__ Fp tm_mul_call(Fp a, Fp b, uint32_t t, uint32_t sm_phase) {
-    {
-        const TmPart x = tm_part(a.v), y = tm_part(b.v);
-        uint32_t z[12];
-        mul_words<6>(z, x.lo, y.lo);
-        tm_put(t, z);
-        mul_words<6>(z, x.hi, y.hi);
-        tm_put(t + 12, z);
-        mul_words<6>(z, x.sum, y.sum);
-        tm_put(t + 24, z);
-    }
-    uint32_t w[kTmCols / 2];
-    tm_exchange(t, sm_phase, w);
-    return tm_result<CANON>(w);
+__device__ __forceinline__ Fp tm_canonical_if(const Fp &a) {
+    if constexpr (CANON) return tm_canonical(a);
+    else return a;
 }
-template <bool CANON>
-__device__ __noinline__ Fp tm_sqr_call(Fp a, uint32_t t, uint32_t sm_phase) {
-    {
-        const TmPart x = tm_part(a.v);
-        uint32_t z[12];
-        sqr_words<6>(z, x.lo);
-        tm_put(t, z);
-        sqr_words<6>(z, x.hi);
-        tm_put(t + 12, z);
-        sqr_words<6>(z, x.sum);
-        tm_put(t + 24, z);
-    }
-    uint32_t w[kTmCols / 2];
-    tm_exchange(t, sm_phase, w);
-    return tm_result<CANON>(w);
+
+// the three Karatsuba products of a b, or of a^2, to the product's byte area
+__device__ __forceinline__ void tm_put_mul(const Fp &a, const Fp &b, uint32_t t, uint32_t ctl) {
+    t += (ctl & 2u) / 2 * kTmBytes;
+    const TmPart x = tm_part(a.v), y = tm_part(b.v);
+    uint32_t z[12];
+    mul_words<6>(z, x.lo, y.lo);
+    tm_put(t, z);
+    mul_words<6>(z, x.hi, y.hi);
+    tm_put(t + 12, z);
+    mul_words<6>(z, x.sum, y.sum);
+    tm_put(t + 24, z);
 }
-// a b and a^2, called by every thread of a group together
+__device__ __forceinline__ void tm_put_sqr(const Fp &a, uint32_t t, uint32_t ctl) {
+    t += (ctl & 2u) / 2 * kTmBytes;
+    const TmPart x = tm_part(a.v);
+    uint32_t z[12];
+    sqr_words<6>(z, x.lo);
+    tm_put(t, z);
+    sqr_words<6>(z, x.hi);
+    tm_put(t + 12, z);
+    sqr_words<6>(z, x.sum);
+    tm_put(t + 24, z);
+}
+__device__ __noinline__ Fp tm_mul_call(Fp a, Fp b, uint32_t t, uint32_t ctl) {
+    tm_put_mul(a, b, t, ctl);
+    tm_start(t, ctl);
+    uint32_t w[kTmCols / 2];
+    tm_sums(t, ctl, w);
+    return tm_result(w);
+}
+__device__ __noinline__ Fp tm_sqr_call(Fp a, uint32_t t, uint32_t ctl) {
+    tm_put_sqr(a, t, ctl);
+    tm_start(t, ctl);
+    uint32_t w[kTmCols / 2];
+    tm_sums(t, ctl, w);
+    return tm_result(w);
+}
+__device__ __noinline__ void tm_push_first_call(Fp a, Fp b, uint32_t t, uint32_t ctl) {
+    tm_put_mul(a, b, t, ctl);
+    tm_start(t, ctl);
+}
+__device__ __noinline__ Fp tm_push_mul_call(Fp a, Fp b, uint32_t t, uint32_t ctl) {
+    tm_put_mul(a, b, t, ctl);
+    uint32_t w[kTmCols / 2];
+    tm_sums(t, ctl, w);
+    tm_start(t, ctl);
+    return tm_result(w);
+}
+__device__ __noinline__ Fp tm_push_sqr_call(Fp a, uint32_t t, uint32_t ctl) {
+    tm_put_sqr(a, t, ctl);
+    uint32_t w[kTmCols / 2];
+    tm_sums(t, ctl, w);
+    tm_start(t, ctl);
+    return tm_result(w);
+}
+__device__ __noinline__ Fp tm_pop_call(uint32_t t, uint32_t ctl) {
+    uint32_t w[kTmCols / 2];
+    tm_sums(t, ctl, w);
+    return tm_result(w);
+}
+
+// a b and a^2, called by every thread of a group together (none in flight)
 template <bool CANON>
 __device__ __forceinline__ Fp tm_mul(Tm &g, const Fp &a, const Fp &b) {
     __syncwarp();
-    const Fp r = tm_mul_call<CANON>(a, b, g.t, g.sm);
+    const Fp r = tm_mul_call(a, b, g.t, g.sm);
     g.sm ^= 1u;
-    return r;
+    return tm_canonical_if<CANON>(r);
 }
 template <bool CANON>
 __device__ __forceinline__ Fp tm_sqr(Tm &g, const Fp &a) {
     __syncwarp();
-    const Fp r = tm_sqr_call<CANON>(a, g.t, g.sm);
+    const Fp r = tm_sqr_call(a, g.t, g.sm);
     g.sm ^= 1u;
-    return r;
+    return tm_canonical_if<CANON>(r);
+}
+
+// The same products in a pipeline of depth one: a push starts a product and
+// returns the one pushed before it, whose trip through the tensor core has run
+// while the new one's words were multiplied; CANON speaks of the one returned.
+// tm_push_first starts the pipeline, tm_pop ends it.
+__device__ __forceinline__ void tm_push_first(Tm &g, const Fp &a, const Fp &b) {
+    __syncwarp();
+    tm_push_first_call(a, b, g.t, g.sm);
+    g.sm ^= 2u;
+}
+template <bool CANON>
+__device__ __forceinline__ Fp tm_push(Tm &g, const Fp &a, const Fp &b) {
+    __syncwarp();
+    const Fp r = tm_push_mul_call(a, b, g.t, g.sm);
+    g.sm ^= 3u;
+    return tm_canonical_if<CANON>(r);
+}
+template <bool CANON>
+__device__ __forceinline__ Fp tm_push_sqr(Tm &g, const Fp &a) {
+    __syncwarp();
+    const Fp r = tm_push_sqr_call(a, g.t, g.sm);
+    g.sm ^= 3u;
+    return tm_canonical_if<CANON>(r);
+}
+template <bool CANON>
+__device__ __forceinline__ Fp tm_pop(Tm &g) {
+    __syncwarp();
+    const Fp r = tm_pop_call(g.t, g.sm);
+    g.sm ^= 1u;
+    return tm_canonical_if<CANON>(r);
 }
 
 // the same products by the scalar multiplier, for kernels that take either
-struct ScalarMul {};
+struct ScalarMul {
+    Fp last; // the product pushed last
+};
 template <bool CANON>
 __device__ __forceinline__ Fp tm_mul(ScalarMul &, const Fp &a, const Fp &b) {
     return fp_mul(a, b);
@@ -398,6 +491,23 @@ __device__ __forceinline__ Fp tm_mul(ScalarMul &, const Fp &a, const Fp &b) {
 template <bool CANON>
 __device__ __forceinline__ Fp tm_sqr(ScalarMul &, const Fp &a) {
     return fp_sqr(a);
+}
+__device__ __forceinline__ void tm_push_first(ScalarMul &g, const Fp &a, const Fp &b) { g.last = fp_mul(a, b); }
+template <bool CANON>
+__device__ __forceinline__ Fp tm_push(ScalarMul &g, const Fp &a, const Fp &b) {
+    const Fp r = g.last;
+    g.last = fp_mul(a, b);
+    return r;
+}
+template <bool CANON>
+__device__ __forceinline__ Fp tm_push_sqr(ScalarMul &g, const Fp &a) {
+    const Fp r = g.last;
+    g.last = fp_sqr(a);
+    return r;
+}
+template <bool CANON>
+__device__ __forceinline__ Fp tm_pop(ScalarMul &g) {
+    return g.last;
 }
 #endif
 
