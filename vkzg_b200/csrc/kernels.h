@@ -215,6 +215,9 @@ void trim_working_set(vkzg_prover *p);
 void set_comb_budget(vkzg_prover *p, uint64_t bytes);
 void precapture_graphs(vkzg_prover *p, uint32_t max_n);
 
+// SMs of the current device
+int sm_count();
+
 // process-wide count of kernels launched by the launchers above
 void count_launches(int k);
 uint64_t launches_total();

@@ -48,6 +48,12 @@ void count_launches(int k) {
     g_launches.fetch_add((uint64_t)(int64_t)k, std::memory_order_relaxed);
     t_launches += (uint64_t)(int64_t)k;
 }
+int sm_count() {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
 uint64_t launches_total() { return g_launches.load(std::memory_order_relaxed); }
 } // namespace vkzg
 
