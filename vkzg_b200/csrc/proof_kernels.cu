@@ -231,6 +231,47 @@ __global__ void __launch_bounds__(kReduceThreads) k_reduce(const G1J *__restrict
     st_vec(&out[o], g1_add(w, acc));
 }
 
+// The same sum with a warp per output, for few outputs: lane l sums buckets
+// [4 l, 4 l + 4) to S_l and W_l, a suffix scan over the lanes gives
+// T_l = sum of S_m, m >= l, with sum_l l S_l = sum of T_l, l >= 1, and the lanes'
+// W_l + 4 T_l add up in a tree: 20 point operations one after another instead of
+// 57, for 2.3 times the work.  Latency is what counts while every output's warp
+// has a scheduler of its own (n_outputs <= 4 SMs): 0.95 ms a reduction with 8
+// lanes at 1 to 4 blobs.
+constexpr int kReduceWarpThreads = 64;
+__global__ void __launch_bounds__(kReduceWarpThreads) k_reduce_warp(const G1J *__restrict__ buckets, G1J *out,
+                                                                  int n_outputs) {
+    const int o = (int)(blockIdx.x * blockDim.x + threadIdx.x) / 32, lane = threadIdx.x & 31;
+    if (o >= n_outputs) return; // whole warps
+    constexpr int per = kBuckets / 32;
+    const G1J *bk = buckets + (size_t)o * kBuckets + lane * per;
+    G1J s = ld_vec(&bk[per - 1]), w = s;
+    for (int k = per - 2; k >= 0; k--) {
+        s = g1_add(s, ld_vec(&bk[k]));
+        w = g1_add(w, s);
+    }
+#pragma unroll 1
+    for (int d = 1; d < 32; d <<= 1) {
+        const G1J other = g1_shfl_down(s, d);
+        if (lane + d < 32) s = g1_add(s, other);
+    }
+    if (lane) w = g1_add(w, g1_dbl(g1_dbl(s)));
+#pragma unroll 1
+    for (int d = 16; d >= 1; d >>= 1) {
+        const G1J other = g1_shfl_down(w, d);
+        if (lane < d) w = g1_add(w, other);
+    }
+    if (lane == 0) st_vec(&out[o], w);
+}
+static void launch_reduce(const G1J *buckets, G1J *out, int n_outputs, cudaStream_t s) {
+    if (n_outputs <= 4 * sm_count())
+        k_reduce_warp<<<(n_outputs * 32 + kReduceWarpThreads - 1) / kReduceWarpThreads, kReduceWarpThreads, 0, s>>>(
+            buckets, out, n_outputs);
+    else
+        k_reduce<<<(n_outputs * kReduceLanes + kReduceThreads - 1) / kReduceThreads, kReduceThreads, 0, s>>>(
+            buckets, out, n_outputs);
+}
+
 // ---------------------------------------------------------------- stages 5-6
 // One block per blob, one thread per point.  First the parts of phase B's
 // convolution (PartLayout) in shared memory: level l folds the cyclic vector v
@@ -254,6 +295,49 @@ __device__ __forceinline__ void butterfly_level(G1J *v, int t, int m) {
     __syncthreads();
     if (t < 2 * m) st_vec(&v[t], r);
     __syncthreads();
+}
+
+// The ladder with four lanes per point and a quarter of a blob's points per block,
+// for few blobs: a doubling's independent products run side by side on the lanes
+// (X^2, Y^2, Y Z; then E^2, B^2, (X + B)^2), three products one after another
+// instead of seven.  Every block folds the whole blob.  While each block has an
+// SM of its own (n <= SMs / 4); with more blobs the lanes would share schedulers.
+constexpr int kLadderSplit = 4;
+__device__ __forceinline__ Fp fp_shfl_lane(const Fp &a, int src) {
+    Fp r;
+#pragma unroll
+    for (int i = 0; i < 12; i++) r.v[i] = __shfl_sync(0xffffffffu, a.v[i], src);
+    return r;
+}
+__global__ void __launch_bounds__(kCells) k_ladder_lanes(const G1J *__restrict__ u, G1J *ladder, int levels) {
+    __shared__ G1J v[kCells];
+    const int b = blockIdx.x / kLadderSplit, t = threadIdx.x;
+    st_vec(&v[t], ld_vec(&u[(size_t)b * kCells + t]));
+    __syncthreads();
+    for (int l = 1; l <= levels; l++) butterfly_level(v, t, kCells >> l);
+    const int point = (int)(blockIdx.x % kLadderSplit) * (kCells / kLadderSplit) + t / 4;
+    const int role = t & 3, base = (t & 31) & ~3; // the point's lanes base..base + 3 of the warp
+    G1J acc = ld_vec(&v[point]);
+    G1J *dst = ladder + ((size_t)b * kCells + point) * kLadderDigits;
+    for (int d = 0; d < kLadderDigits; d++) {
+        if (role == 0) st_vec(&dst[d], acc);
+        if (d + 1 == kLadderDigits) break;
+#pragma unroll 1
+        for (int q = 0; q < 8; q++) { // 2 acc; infinity (Z = 0) stays: Z3 = 2 Y Z = 0
+            Fp r = fp_mul(role == 0 ? acc.x : acc.y, role == 0 ? acc.x : role == 1 ? acc.y : acc.z);
+            const Fp A = fp_shfl_lane(r, base), B = fp_shfl_lane(r, base + 1), YZ = fp_shfl_lane(r, base + 2);
+            const Fp E = fp_add(fp_dbl(A), A);
+            r = fp_sqr(role == 0 ? E : role == 1 ? B : fp_add(acc.x, B));
+            const Fp F = fp_shfl_lane(r, base), C = fp_shfl_lane(r, base + 1), XB = fp_shfl_lane(r, base + 2);
+            const Fp D = fp_dbl(fp_sub(fp_sub(XB, A), C));
+            const Fp x3 = fp_sub(F, fp_dbl(D));
+            const Fp y3 = fp_sub(fp_mul(E, fp_sub(D, x3)), fp_dbl(fp_dbl(fp_dbl(C))));
+            const bool inf = fp_is_zero(acc.z); // g1_dbl leaves such a point as it is
+            acc.x = inf ? acc.x : x3;
+            acc.y = inf ? acc.y : y3;
+            acc.z = fp_dbl(YZ);
+        }
+    }
 }
 
 __global__ void __launch_bounds__(kCells) k_ladder(const G1J *__restrict__ u, G1J *ladder, int levels) {
@@ -2307,6 +2391,26 @@ __global__ void __launch_bounds__(128) k_flatr_horner(FlatRArgs a, G1J *out) {
     st_vec(&out[o], red_horner([&](int x) { return ld_vec(red_slot(a, o, x)); }));
 }
 
+// The Horner step with eight lanes per output, one per term: lane j adds up its
+// term's slots (at most 4), doubles the sum j times (S, lane 7, none), and the
+// lanes add up in a tree: 123 products one after another instead of 317.
+__global__ void __launch_bounds__(64) k_flatr_terms(FlatRArgs a, G1J *out) {
+    const uint32_t gl = blockIdx.x * blockDim.x + threadIdx.x, o = gl >> 3;
+    const int j = (int)(gl & 7u);
+    if (o >= (uint32_t)a.n_out) return; // n_out is a multiple of 128: whole warps
+    G1J h = g1_identity();
+    for (int k = 0; k < c_red.term_n[j]; k++) h = g1_madd(h, ld_vec(red_slot(a, o, c_red.term_slot[j][k])));
+    for (int q = 0; q < (j == 7 ? 0 : j); q++) h = g1_dbl(h);
+    __syncwarp();
+#pragma unroll 1
+    for (int d = 4; d >= 1; d >>= 1) {
+        const G1J other = g1_shfl_down(h, d);
+        if (j < d) h = g1_add(h, other);
+        __syncwarp();
+    }
+    if (j == 0) st_vec(&out[o], h);
+}
+
 // Phase B's Horner step and stage 9 in one launch (plans 3-4): a block is one
 // blob and its 128 threads the blob's outputs, so each thread's Horner result
 // goes to shared memory for the unfolding instead of through HBM.
@@ -2378,7 +2482,13 @@ int launch_reduce_flat(const ProofWork &w, const G1A *buckets, G1J *out, int n_o
         }
         launched += 3 * rounds;
     }
-    if (proofs) k_finish_horner<<<n_out / kCells, kCells, 0, s>>>(a, proofs, kPartLevels);
+    // one thread per output is a chain of 317 products: while eight lanes an
+    // output make at most two warps a scheduler, the eight-lane form is shorter
+    if (proofs && n_out <= 32 * sm_count()) {
+        k_flatr_terms<<<n_out * 8 / 64, 64, 0, s>>>(a, w.points);
+        k_finish<<<n_out / kCells, kCells, 0, s>>>(w.points, proofs, kPartLevels);
+        launched++;
+    } else if (proofs) k_finish_horner<<<n_out / kCells, kCells, 0, s>>>(a, proofs, kPartLevels);
     else k_flatr_horner<<<(n_out + 127) / 128, 128, 0, s>>>(a, out);
     return launched;
 }
@@ -2549,7 +2659,7 @@ cudaError_t launch_proofs_timed(const DeviceTables &t, const ProofWork &w, int n
     const int ba_grid = std::min(w.ba_blocks, (n_out / kWarpOutputs + kBAWarps - 1) / kBAWarps);
     auto reduce = [&](uint8_t *proofs) {
         if (flatb) launched += launch_reduce_flat(w, w.bucket_aff, w.points, n_out, s, proofs) - 1;
-        else if (!affine) k_reduce<<<red_blocks, kReduceThreads, 0, s>>>(w.buckets, w.points, n_out);
+        else if (!affine) launch_reduce(w.buckets, w.points, n_out, s);
         else if (hier)
             k_reduce_hier<<<(n_out + kRedOutputs - 1) / kRedOutputs, kRedThreads, 0, s>>>(w.bucket_aff, w.points,
                                                                                        w.red_scratch, n_out);
@@ -2574,7 +2684,10 @@ cudaError_t launch_proofs_timed(const DeviceTables &t, const ProofWork &w, int n
     // halves; the fold (stage 5) runs inside the ladder's launch
     const int levels = flatb ? kPartLevels : 1;
     mark();
-    k_ladder<<<n, kCells, 0, s>>>(w.points, w.ladder, levels);
+    if (kLadderSplit * n <= sm_count())
+        k_ladder_lanes<<<kLadderSplit * n, kCells, 0, s>>>(w.points, w.ladder, levels);
+    else
+        k_ladder<<<n, kCells, 0, s>>>(w.points, w.ladder, levels);
     mark();
     if (flatb) launched += launch_normalize_flat(w, n, s) - 1;
     else k_normalize<<<(n_lad + kNormThreads - 1) / kNormThreads, kNormThreads, 0, s>>>(w.ladder, w.ladder_aff, n_lad);
