@@ -239,17 +239,21 @@ __global__ void __launch_bounds__(kReduceThreads) k_reduce(const G1J *__restrict
 // has a scheduler of its own (n_outputs <= 4 SMs): 0.95 ms a reduction with 8
 // lanes at 1 to 4 blobs.
 constexpr int kReduceWarpThreads = 64;
-__global__ void __launch_bounds__(kReduceWarpThreads) k_reduce_warp(const G1J *__restrict__ buckets, G1J *out,
+__device__ __forceinline__ G1J reduce_add(const G1J &a, const G1J &b) { return g1_add(a, b); }
+__device__ __forceinline__ G1J reduce_add(const G1J &a, const G1A &b) { return g1_madd(a, b); }
+template <class Point>
+__global__ void __launch_bounds__(kReduceWarpThreads) k_reduce_warp(const Point *__restrict__ buckets, G1J *out,
                                                                   int n_outputs) {
     const int o = (int)(blockIdx.x * blockDim.x + threadIdx.x) / 32, lane = threadIdx.x & 31;
     if (o >= n_outputs) return; // whole warps
     constexpr int per = kBuckets / 32;
-    const G1J *bk = buckets + (size_t)o * kBuckets + lane * per;
-    G1J s = ld_vec(&bk[per - 1]), w = s;
+    const Point *bk = buckets + (size_t)o * kBuckets + lane * per;
+    G1J s = reduce_add(g1_identity(), ld_vec(&bk[per - 1])), w = s;
     for (int k = per - 2; k >= 0; k--) {
-        s = g1_add(s, ld_vec(&bk[k]));
+        s = reduce_add(s, ld_vec(&bk[k]));
         w = g1_add(w, s);
     }
+    __syncwarp();
 #pragma unroll 1
     for (int d = 1; d < 32; d <<= 1) {
         const G1J other = g1_shfl_down(s, d);
@@ -263,10 +267,13 @@ __global__ void __launch_bounds__(kReduceWarpThreads) k_reduce_warp(const G1J *_
     }
     if (lane == 0) st_vec(&out[o], w);
 }
+template <class Point>
+static void launch_reduce_warp(const Point *buckets, G1J *out, int n_outputs, cudaStream_t s) {
+    k_reduce_warp<Point><<<(n_outputs * 32 + kReduceWarpThreads - 1) / kReduceWarpThreads, kReduceWarpThreads, 0, s>>>(
+        buckets, out, n_outputs);
+}
 static void launch_reduce(const G1J *buckets, G1J *out, int n_outputs, cudaStream_t s) {
-    if (n_outputs <= 4 * sm_count())
-        k_reduce_warp<<<(n_outputs * 32 + kReduceWarpThreads - 1) / kReduceWarpThreads, kReduceWarpThreads, 0, s>>>(
-            buckets, out, n_outputs);
+    if (n_outputs <= 4 * sm_count()) launch_reduce_warp(buckets, out, n_outputs, s);
     else
         k_reduce<<<(n_outputs * kReduceLanes + kReduceThreads - 1) / kReduceThreads, kReduceThreads, 0, s>>>(
             buckets, out, n_outputs);
@@ -739,9 +746,9 @@ __device__ __forceinline__ void flat_pass1_products(G &g, const Fp &acc, Fp *oth
 #pragma unroll 1
     for (int d = 2; d < 32; d <<= 1) {
         const Fp partner = fp_shfl_xor(group, d);
-        tm_push_first(g, rest, partner);
-        rest = tm_push<false>(g, group, partner);
-        group = tm_pop<true>(g);
+        tm_push_first(g, group, partner); // the next level waits for this one
+        group = tm_push<true>(g, rest, partner);
+        rest = tm_pop<false>(g);
     }
     st_vec(&others[gl], rest);
     if (lane == 0) st_vec(&tot[wg], group);
@@ -1230,31 +1237,44 @@ __global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSM) k_flat_pass2(F
     tm_end(tm_area, a.err, a.n_err);
 }
 
-// The last m <= kTreeTail points of each list (affine, left by the tree
-// rounds) summed in Jacobian form: the rounds below that length cost an
-// inversion launch each for little work.  Two threads per list, each a chain of
-// mixed additions over alternate points, then one addition.
-constexpr uint32_t kTreeTail = 10;
-// thread t of the tail: half t & 1 of list t >> 1 (all 32 lanes of a warp call
-// it together: the halves meet by a shuffle)
-__device__ __forceinline__ void flat_finish_body(const G1A *lists, uint32_t m, G1J *points, int n, int t) {
-    const int o = t >> 1, h = t & 1;
+// The last points of each list (affine, left by the tree rounds) summed in
+// Jacobian form: the rounds below that length cost three launches each, an
+// inversion among them (70 us together even for a few lists), for little work.
+// T threads per list, each a chain of mixed additions over every T-th point, then
+// a tree over the T.  Two threads and at most 10 points for many lists; while the
+// threads make at most two warps a scheduler, 8 threads and 24 points (32 SMs
+// lists) or a warp and 96 points (8 SMs lists) replace one and three rounds more:
+// 6 blobs 8 rounds and 43 us -> 4 rounds.
+constexpr uint32_t kTreeTail = 10, kTreeTail8 = 24, kTreeTail32 = 96;
+static int tail_threads(int lists) {
+    const int sms = sm_count();
+    return lists <= 8 * sms ? 32 : lists <= 32 * sms ? 8 : 2;
+}
+static uint32_t tail_points(int threads) {
+    return threads == 32 ? kTreeTail32 : threads == 8 ? kTreeTail8 : kTreeTail;
+}
+template <int T>
+__global__ void __launch_bounds__(64) k_flat_finish(const G1A *__restrict__ lists, uint32_t m, G1J *points, int n) {
+    const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x), o = t / T, h = t % T;
     G1J acc = g1_identity();
     if (o < n) {
         const G1A *l = lists + (size_t)o * m;
-        for (uint32_t k = h; k < m; k += 2) acc = g1_madd(acc, ld_vec(&l[k]));
+        for (uint32_t k = h; k < m; k += T) acc = g1_madd(acc, ld_vec(&l[k]));
     }
-    G1J other;
-#pragma unroll
-    for (int w = 0; w < 12; w++) {
-        other.x.v[w] = __shfl_xor_sync(0xffffffffu, acc.x.v[w], 1);
-        other.y.v[w] = __shfl_xor_sync(0xffffffffu, acc.y.v[w], 1);
-        other.z.v[w] = __shfl_xor_sync(0xffffffffu, acc.z.v[w], 1);
+    __syncwarp();
+#pragma unroll 1
+    for (int d = T / 2; d >= 1; d >>= 1) { // the lanes of a warp go through it together
+        const G1J other = g1_shfl_down(acc, d);
+        if (h < d) acc = g1_add(acc, other);
+        __syncwarp();
     }
-    if (o < n && h == 0) st_vec(&points[o], g1_add(acc, other));
+    if (o < n && h == 0) st_vec(&points[o], acc);
 }
-__global__ void __launch_bounds__(64) k_flat_finish(const G1A *__restrict__ lists, uint32_t m, G1J *points, int n) {
-    flat_finish_body(lists, m, points, n, (int)(blockIdx.x * blockDim.x + threadIdx.x));
+static void launch_flat_finish(int threads, const G1A *lists, uint32_t m, G1J *points, int n, cudaStream_t s) {
+    const int blocks = (int)(((size_t)threads * n + 63) / 64);
+    if (threads == 32) k_flat_finish<32><<<blocks, 64, 0, s>>>(lists, m, points, n);
+    else if (threads == 8) k_flat_finish<8><<<blocks, 64, 0, s>>>(lists, m, points, n);
+    else k_flat_finish<2><<<blocks, 64, 0, s>>>(lists, m, points, n);
 }
 
 int flat_blocks() { return sm_count() * kFlatBlocksPerSM; }
@@ -1483,6 +1503,8 @@ int launch_phase_a_flat(const ProofWork &w, int n, cudaStream_t s) {
     a.n_lists = lists;
     a.err = w.err;
     a.n_err = (uint32_t)n;
+    const int tail = tail_threads(lists);
+    const uint32_t stop = tail_points(tail);
     int launched = 0;
     uint32_t m = (uint32_t)L;
     const G1A *res;
@@ -1493,19 +1515,19 @@ int launch_phase_a_flat(const ProofWork &w, int n, cudaStream_t s) {
         launch_coop(k_coop_tree<true>, w.flat_blocks, kStage2Bytes, s, a, (const G1A *)nullptr, w.flat_buf[0],
                     w.flat_buf[1], m0, (m0 + 1) >> 1, make_sync(w, n));
         launched++;
-        if (((m0 + 1) >> 1) > kTreeTail) {
+        if (((m0 + 1) >> 1) > stop) {
             launch_coop(k_coop_tree<false>, w.flat_blocks, kStage2Bytes, s, a, (const G1A *)w.flat_buf[0], w.flat_buf[1],
-                        w.flat_buf[0], (m0 + 1) >> 1, kTreeTail, make_sync(w, n));
+                        w.flat_buf[0], (m0 + 1) >> 1, stop, make_sync(w, n));
             launched++;
         }
-        res = tree_result(nullptr, &m, kTreeTail, w.flat_buf[0], w.flat_buf[1]);
+        res = tree_result(nullptr, &m, stop, w.flat_buf[0], w.flat_buf[1]);
     } else {
         k_flat_digits<<<lists * kCellElems / 128, 128, 0, s>>>(w.scalars, w.flat_dig, a.win, lists * kCellElems);
         launched++;
-        res = run_tree_rounds<true>(a, nullptr, &m, kTreeTail, w.flat_buf[0], w.flat_buf[1], w.flat_blocks, s,
+        res = run_tree_rounds<true>(a, nullptr, &m, stop, w.flat_buf[0], w.flat_buf[1], w.flat_blocks, s,
                                     &launched);
     }
-    k_flat_finish<<<(2 * lists + 63) / 64, 64, 0, s>>>(res, m, w.points, lists);
+    launch_flat_finish(tail, res, m, w.points, lists, s);
     return launched + 1;
 }
 
@@ -2459,6 +2481,14 @@ int launch_reduce_flat(const ProofWork &w, const G1A *buckets, G1J *out, int n_o
         ReduceSchedule h;
         return build_reduce_schedule(h) ? h.n_rounds : 0;
     }();
+    // for few outputs the rounds' launches and the Horner chain take longer than
+    // a warp per output (k_reduce_warp), up to two warps a scheduler
+    if (n_out <= 8 * sm_count() && !w.coop) {
+        launch_reduce_warp(buckets, proofs ? w.points : out, n_out, s);
+        if (!proofs) return 1;
+        k_finish<<<n_out / kCells, kCells, 0, s>>>(w.points, proofs, kPartLevels);
+        return 2;
+    }
     FlatRArgs a;
     a.buckets = buckets;
     a.slots = w.red_scratch;
