@@ -304,42 +304,56 @@ __device__ __forceinline__ void butterfly_level(G1J *v, int t, int m) {
     __syncthreads();
 }
 
-// The ladder with four lanes per point and a quarter of a blob's points per block,
-// for few blobs: a doubling's independent products run side by side on the lanes
-// (X^2, Y^2, Y Z; then E^2, B^2, (X + B)^2), three products one after another
-// instead of seven.  Every block folds the whole blob.  While each block has an
-// SM of its own (n <= SMs / 4); with more blobs the lanes would share schedulers.
-constexpr int kLadderSplit = 4;
+// The ladder with LANES lanes per point, for fewer blobs than fill the GPU: a
+// doubling's independent products run side by side on a point's lanes.  Four
+// lanes (and a quarter of a blob's points per block): X^2, Y^2, Y Z, then E^2, B^2,
+// (X + B)^2, then Y3's product: three one after another instead of seven.  Two
+// lanes (half of the points): X^2 and Y^2, Y Z and B^2, E^2 and (X + B)^2, then Y3's:
+// four.  Every block folds the whole blob.  Each while a block has an SM of its
+// own (n <= SMs / LANES); with more blobs the lanes would share schedulers.
 __device__ __forceinline__ Fp fp_shfl_lane(const Fp &a, int src) {
     Fp r;
 #pragma unroll
     for (int i = 0; i < 12; i++) r.v[i] = __shfl_sync(0xffffffffu, a.v[i], src);
     return r;
 }
+template <int LANES>
 __global__ void __launch_bounds__(kCells) k_ladder_lanes(const G1J *__restrict__ u, G1J *ladder, int levels) {
+    static_assert(LANES == 2 || LANES == 4, "two or four lanes a point");
     __shared__ G1J v[kCells];
-    const int b = blockIdx.x / kLadderSplit, t = threadIdx.x;
+    const int b = blockIdx.x / LANES, t = threadIdx.x;
     st_vec(&v[t], ld_vec(&u[(size_t)b * kCells + t]));
     __syncthreads();
     for (int l = 1; l <= levels; l++) butterfly_level(v, t, kCells >> l);
-    const int point = (int)(blockIdx.x % kLadderSplit) * (kCells / kLadderSplit) + t / 4;
-    const int role = t & 3, base = (t & 31) & ~3; // the point's lanes base..base + 3 of the warp
+    const int point = (int)(blockIdx.x % LANES) * (kCells / LANES) + t / LANES;
+    const int role = t % LANES, base = (t & 31) - role; // the point's lanes base.. of the warp
     G1J acc = ld_vec(&v[point]);
     G1J *dst = ladder + ((size_t)b * kCells + point) * kLadderDigits;
     for (int d = 0; d < kLadderDigits; d++) {
         if (role == 0) st_vec(&dst[d], acc);
         if (d + 1 == kLadderDigits) break;
 #pragma unroll 1
-        for (int q = 0; q < 8; q++) { // 2 acc; infinity (Z = 0) stays: Z3 = 2 Y Z = 0
-            Fp r = fp_mul(role == 0 ? acc.x : acc.y, role == 0 ? acc.x : role == 1 ? acc.y : acc.z);
-            const Fp A = fp_shfl_lane(r, base), B = fp_shfl_lane(r, base + 1), YZ = fp_shfl_lane(r, base + 2);
-            const Fp E = fp_add(fp_dbl(A), A);
-            r = fp_sqr(role == 0 ? E : role == 1 ? B : fp_add(acc.x, B));
-            const Fp F = fp_shfl_lane(r, base), C = fp_shfl_lane(r, base + 1), XB = fp_shfl_lane(r, base + 2);
+        for (int q = 0; q < 8; q++) { // 2 acc
+            Fp A, B, C, YZ, E, F, XB;
+            if constexpr (LANES == 4) {
+                Fp r = fp_mul(role == 0 ? acc.x : acc.y, role == 0 ? acc.x : role == 1 ? acc.y : acc.z);
+                A = fp_shfl_lane(r, base), B = fp_shfl_lane(r, base + 1), YZ = fp_shfl_lane(r, base + 2);
+                E = fp_add(fp_dbl(A), A);
+                r = fp_sqr(role == 0 ? E : role == 1 ? B : fp_add(acc.x, B));
+                F = fp_shfl_lane(r, base), C = fp_shfl_lane(r, base + 1), XB = fp_shfl_lane(r, base + 2);
+            } else {
+                Fp r = fp_sqr(role == 0 ? acc.x : acc.y);
+                A = fp_shfl_lane(r, base), B = fp_shfl_lane(r, base + 1);
+                r = fp_mul(role == 0 ? acc.y : B, role == 0 ? acc.z : B);
+                YZ = fp_shfl_lane(r, base), C = fp_shfl_lane(r, base + 1);
+                E = fp_add(fp_dbl(A), A);
+                r = fp_sqr(role == 0 ? E : fp_add(acc.x, B));
+                F = fp_shfl_lane(r, base), XB = fp_shfl_lane(r, base + 1);
+            }
             const Fp D = fp_dbl(fp_sub(fp_sub(XB, A), C));
             const Fp x3 = fp_sub(F, fp_dbl(D));
             const Fp y3 = fp_sub(fp_mul(E, fp_sub(D, x3)), fp_dbl(fp_dbl(fp_dbl(C))));
-            const bool inf = fp_is_zero(acc.z); // g1_dbl leaves such a point as it is
+            const bool inf = fp_is_zero(acc.z); // g1_dbl leaves such a point as it is; Z3 = 2 Y Z = 0
             acc.x = inf ? acc.x : x3;
             acc.y = inf ? acc.y : y3;
             acc.z = fp_dbl(YZ);
@@ -2714,8 +2728,11 @@ cudaError_t launch_proofs_timed(const DeviceTables &t, const ProofWork &w, int n
     // halves; the fold (stage 5) runs inside the ladder's launch
     const int levels = flatb ? kPartLevels : 1;
     mark();
-    if (kLadderSplit * n <= sm_count())
-        k_ladder_lanes<<<kLadderSplit * n, kCells, 0, s>>>(w.points, w.ladder, levels);
+    const int sms = sm_count();
+    if (4 * n <= sms)
+        k_ladder_lanes<4><<<4 * n, kCells, 0, s>>>(w.points, w.ladder, levels);
+    else if (2 * n <= sms)
+        k_ladder_lanes<2><<<2 * n, kCells, 0, s>>>(w.points, w.ladder, levels);
     else
         k_ladder<<<n, kCells, 0, s>>>(w.points, w.ladder, levels);
     mark();
