@@ -50,6 +50,9 @@ RECOVERY_IMAD_PER_BLOB = 118e6       # 0.46M Fr mul (4 NTT-8192 + pointwise + ba
 NOMINAL_IMAD_TPS = 148 * 64 * 1.965e9 / 1e12
 # this library's Fp product (one Karatsuba level + word-serial reduction) and square
 IMAD_FP_MUL_KS, IMAD_FP_SQR_KS = 516, 426
+# the same reduced on the tensor cores, as the grid-wide rounds make them: 108 (63
+# for a square) and 12 word products of two multiply instructions, and one more
+IMAD_FP_MUL_TM, IMAD_FP_SQR_TM = 241, 151
 PHASE_A_TAIL = 10  # lists of at most this many points finish in Jacobian form
 
 
@@ -67,18 +70,17 @@ def phase_a_executed_products_per_output(d):
 
 def phase_a_executed_imad_per_output(d):
     """Multiply instructions plan 3's phase A executes per MSM output with d
-    windows: affine additions (5 products + 1 square) in tree rounds down to
-    lists of PHASE_A_TAIL points, then mixed additions (7 + 4) on two chains and
-    one Jacobian addition (11 + 5)."""
+    windows: affine additions (5 products + 1 square, reduced on the tensor cores)
+    in tree rounds down to lists of PHASE_A_TAIL points, then mixed additions
+    (7 + 4) on two chains and one Jacobian addition (11 + 5)."""
     m = 64 * d
     adds = 0
     while m > PHASE_A_TAIL:
         adds += m // 2
         m = (m + 1) // 2
     madds = max(m - 2, 0)
-    muls = 5 * adds + 7 * madds + 11
-    sqrs = adds + 4 * madds + 5
-    return muls * IMAD_FP_MUL_KS + sqrs * IMAD_FP_SQR_KS
+    return (adds * (5 * IMAD_FP_MUL_TM + IMAD_FP_SQR_TM) + (7 * madds + 11) * IMAD_FP_MUL_KS +
+            (4 * madds + 5) * IMAD_FP_SQR_KS)
 
 
 def phase_a_dram_bytes(d, n_blobs):
@@ -664,7 +666,7 @@ def run_ours(args, rank, world, local_rank):
 
     # ---- roofline of the dominant kernel (phase A), integer-multiply bound
     imad_peak = vkzg_b200.microbench(0)
-    product_rate = vkzg_b200.microbench(4)  # this library's Fp product alone, G/s
+    product_rate = vkzg_b200.microbench(4)  # this library's scalar Fp product alone, G/s
     pa_ms = statistics.mean(phase_a_ms)
     reference_work = PHASE_A_FP_MUL_PER_BLOB * IMAD_FP * n / (pa_ms / 1e3) / 1e12
     digit = prover.digit_table()
@@ -726,7 +728,8 @@ def run_ours(args, rank, world, local_rank):
                                     f"1.965 GHz = {NOMINAL_IMAD_TPS:.1f}",
                      "algorithmic": "multiply instructions phase A executes: per MSM output 64 D - 1 (D windows) "
                                     "digit-table points summed by affine additions (5 products + 1 square, "
-                                    "516 / 426 multiply instructions each) down to lists of 10, then mixed "
+                                    "241 / 151 multiply instructions each, their reduction on the tensor cores) "
+                                    "down to lists of 10, then mixed "
                                     "Jacobian additions",
                      "products_g_per_s": products, "product_rate_alone_g_per_s": product_rate,
                      "frac_of_product_rate": products / product_rate if products else None,

@@ -67,7 +67,7 @@ vkzg_result vkzg_b200_recover_cells_device(vkzg_prover *p, uint8_t *d_cells_out,
  * fail), latency-critical loops that cannot absorb the device-wide
  * synchronisation a cudaMalloc/cudaFree can imply, and code that enqueues work
  * on a stream it does not own.  This call allocates nothing and frees nothing,
- * and uses no scratch: one cluster of four blocks per blob keeps its working
+ * and uses no scratch: one cluster of blocks per blob keeps its working
  * state in shared memory.  Inputs and outputs are the caller's device buffers,
  * laid out as for vkzg_b200_recover_cells_device; the work is enqueued on
  * `stream` (a cudaStream_t, NULL = legacy default stream) and the call returns

@@ -1,13 +1,14 @@
 // FK20 cell-proof pipeline (reference: src/vkzg.cpp:899-1039 and the k_*.comp
 // kernels it dispatches).  Stages:
-//   1 k_blob_to_coeffs   blob bytes -> Fr, canonicity flag, inverse NTT-4096 in
-//                        shared memory, x 1/4096            (k_blob_to_fr, k_ntt_pass x2)
+//   1 k_blob_to_coeffs   blob bytes -> Fr, canonicity flag, inverse NTT-4096 in a
+//                        cluster's shared memory, x 1/4096  (k_blob_to_fr, k_ntt_pass x2)
 //   2 k_circulant        64 circulant columns, forward NTT-128, canonical
 //                        scalars coeffs[j][i]               (k_build_circulant)
 //   3 k_phase_a          per output j: signed-digit recode, bucket sort in
 //                        shared memory, fixed-base bucket accumulation over the
 //                        position table                     (k_phase_a_sort, k_phase_a)
-//   4 k_reduce           sum_k k * B_k, 8 lanes per output  (k_bucket_reduce)
+//   4 k_reduce           sum_k k * B_k, 8 lanes per output, or a warp for few
+//                        outputs (k_reduce_warp)            (k_bucket_reduce)
 //   5 k_ladder (fold)    u+- = u[j] +- u[j+64], and for plans 3-4 twice more on
 //                        the cyclic half: the convolution's parts (k_fold_ladder)
 //   6 k_ladder           L[j][d] = 2^(8d) v[j], d < 16      (k_ladder, d < 32: the

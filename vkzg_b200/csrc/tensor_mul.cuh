@@ -17,7 +17,13 @@
 //
 // What bounds it: issue slots.  A fused wide multiply-add holds a scheduler
 // about four cycles and every other instruction one; the word-serial form spends
-// 264 of the former per product, this one 120.
+// 264 of the former per product, this one 120.  Measured on B200, two blocks of 256
+// threads per SM: products 41.7 to 42.5 G/s one after another and 42.3 (warps
+// counted in) to 45.3 (a barrier per product) in the pipeline below, against 28.7
+// G/s for the scalar form; squares 51 and 52 to 55 against 33.1.  The matrix
+// product takes 48 cycles of an SM per step of 32 rows.  Tried and slower: the
+// reduction through mma.sync (26.8 G/s), products of 24-bit limbs on the FP64 pipe
+// (25.9) or of 30-bit limbs without carries (29.8) in front of the same reduction.
 #pragma once
 
 #include "field.cuh"
