@@ -45,9 +45,10 @@ def reference_dir(arg=None):
 
 
 def build(ref=None, force=False):
-    """Compiles both programs; returns their paths, or None when no checkout is given."""
+    """Compiles both programs; returns their paths, or None when no checkout is
+    given (an empty directory is none)."""
     ref = reference_dir(ref)
-    if not ref or not os.path.isdir(ref):
+    if not ref or not all(os.path.exists(os.path.join(ref, s)) for _, srcs in PROGRAMS for s in srcs):
         return None
     lib = os.path.join(LIBDIR, "libvkzg.so")
     if not os.path.exists(lib):
