@@ -50,3 +50,45 @@ def test_cooperative_rounds_match_round_launches(monkeypatch, plan):
             outs[coop] = out
     assert np.array_equal(outs["1"], outs["0"])
     assert launches["1"] <= 10 < launches["0"]
+
+
+def test_failed_chunk_is_reported_by_every_entry_point(monkeypatch):
+    """Grid barriers that give up at once ($VKZG_SYNC_POLLS=0): every call that makes
+    proofs reports the failure and leaves no proof in the output, recovery alone
+    is unaffected, and a prover without the limit works in the same process."""
+    torch = pytest.importorskip("torch")
+    monkeypatch.delenv("VKZG_TABLES_PATH", raising=False)
+    monkeypatch.setenv("VKZG_PLAN", "3")
+    monkeypatch.setenv("VKZG_COMB_BITS", "9")
+    n = 3
+    blobs = random_blobs(n, 809)
+    cells, want = np.zeros(n * 262144, np.uint8), np.zeros(n * 6144, np.uint8)
+    present = np.ones((n, 128), np.uint8)
+    present[:, ::2] = 0
+    with vkzg_b200.Prover(max_batch_size=4) as p:
+        assert p.compute_cells_and_proofs_raw(cells, want, blobs, n) == 0
+    erased = cells.reshape(n, 128, 2048) * present[:, :, None]
+    out, got = np.zeros_like(cells), np.zeros_like(want)
+    with monkeypatch.context() as m:
+        m.setenv("VKZG_COOP", "1")
+        m.setenv("VKZG_SYNC_POLLS", "0")
+        with vkzg_b200.Prover(max_batch_size=4) as p:
+            assert p.compute_proofs_raw(got, blobs, n) == vkzg_b200.ERR_GPU
+            assert not got.any()
+            assert p.compute_cells_and_proofs_raw(out, got, blobs, n) == vkzg_b200.ERR_GPU
+            assert not got.any() and not out.any()
+            assert p.recover_cells_and_proofs_raw(out, got, erased, present, n) == vkzg_b200.ERR_GPU
+            assert not got.any()
+            dev = torch.device("cuda", 0)
+            d_in, d_out = torch.from_numpy(blobs.reshape(-1).copy()).to(dev), torch.zeros(n * 6144, dtype=torch.uint8, device=dev)
+            d_err = torch.zeros(n, dtype=torch.int32, device=dev)
+            assert p.compute_proofs_device(d_out.data_ptr(), d_in.data_ptr(), d_err.data_ptr(), n,
+                                           torch.cuda.current_stream(dev).cuda_stream) == 0
+            assert (d_err.cpu().numpy() < 0).all()  # bit 31
+            out[:] = 0
+            assert p.recover_cells_raw(out, erased, present, n) == 0
+            assert np.array_equal(out, cells)
+    with vkzg_b200.Prover(max_batch_size=4) as p:
+        out[:] = 0
+        assert p.recover_cells_and_proofs_raw(out, got, erased, present, n) == 0
+    assert np.array_equal(out, cells) and np.array_equal(got, want)

@@ -145,6 +145,8 @@ struct ProofWork {
     // (grid barriers between passes) when true, else three launches per round
     bool coop = false;
     uint32_t *sync = nullptr;   // [4] grid-barrier words of the cooperative launches
+    // polls of a grid barrier before it gives up: far above any round's duration
+    uint32_t sync_polls = 1u << 24;
 };
 // Batch-affine kernels: VKZG_BA_THREADS threads per block, one warp sums the
 // buckets of kWarpOutputs MSM outputs at a time.  Per-warp scratch: round-1 and

@@ -1483,15 +1483,12 @@ cudaError_t launch_coop(void (*kernel)(KArgs...), int blocks, size_t smem, cudaS
     return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-// polls of a grid barrier before it gives up: far above any round's duration
-constexpr uint32_t kSyncSpinLimit = 1u << 24;
-
 GridSync make_sync(const ProofWork &w, int n) {
     GridSync g;
     g.word = w.sync;
     g.err = w.err;
     g.n_err = (uint32_t)n;
-    g.spin_limit = kSyncSpinLimit;
+    g.spin_limit = w.sync_polls;
     g.expected = (uint32_t)w.flat_blocks;
     return g;
 }

@@ -836,6 +836,7 @@ void take_comb(ProofWork &w, const ProofWork &from) {
     w.deriv_buf = from.deriv_buf;
     w.coop = from.coop;
     w.sync = from.sync;
+    w.sync_polls = from.sync_polls;
 }
 
 // The proof pipeline of one chunk on the prover's own working set (p->pw with
@@ -947,6 +948,9 @@ bool ensure_flat_b(vkzg_prover *p) {
     if (!p->coop_off && coop && atoi(coop) != 0 && coop_supported(z.blocks / (int)p->sm_count) &&
         p->alloc(w.sync, 4))
         w.coop = true;
+    // $VKZG_SYNC_POLLS: the grid barriers' poll limit (0: every wait gives up, for
+    // tests of what callers see then)
+    if (const char *e = getenv("VKZG_SYNC_POLLS")) w.sync_polls = (uint32_t)strtoul(e, nullptr, 10);
     cudaGetLastError();
     return true;
 }
@@ -1999,10 +2003,17 @@ vkzg_result vkzg_b200_recover_cells_and_proofs_batch(vkzg_prover *p, uint8_t *ce
         CK(cudaMemsetAsync(p->pw.err, 0, n * sizeof(uint32_t), s));
         p->pw.plan = plan_for(p, n);
         CK(run_proofs(p, p->pw, n));
+        CK(cudaMemcpyAsync(p->h_err, p->pw.err, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
         CK(cudaMemcpyAsync(cells_out + done * ext_bytes, p->rw.out, (size_t)n * ext_bytes, cudaMemcpyDeviceToHost, s));
-        CK(cudaMemcpyAsync(proofs_out + done * kCells * kProofBytes, p->pw.proofs, (size_t)n * kCells * kProofBytes,
-                           cudaMemcpyDeviceToHost, s));
+        uint8_t *proofs = proofs_out + done * kCells * kProofBytes;
+        CK(cudaMemcpyAsync(proofs, p->pw.proofs, (size_t)n * kCells * kProofBytes, cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
+        // a wait of the proof kernels gave up: the chunk's proofs are not proofs
+        for (uint32_t b = 0; b < n; b++) {
+            if (!(p->h_err[b] & kSyncFailed)) continue;
+            memset(proofs, 0, (size_t)n * kCells * kProofBytes);
+            return VKZG_ERR_GPU;
+        }
         done += n;
     }
     return VKZG_OK;
