@@ -281,6 +281,19 @@ vkzg_result vkzg_b200_grid_sync_selftest(uint32_t extra_arrivals, uint32_t spin_
 vkzg_result vkzg_b200_inverse_selftest(int n, uint32_t seed, uint32_t *mismatched_words);
 
 /*
+ * Self-test of the Fp products reduced on the tensor cores, on n pairs of
+ * operands below 2^382 (12 words each, least significant first).  results: five
+ * arrays of n values, all over 2^384 mod p: a b and a^2 made one after another,
+ * below p + 2^365, then a b, b^2 and a^2 through the pipeline, below p.
+ * give_up != 0: afterwards every warp waits for a product that was never
+ * started; the wait gives up (after some tens of milliseconds), the launch ends
+ * and *error_words_marked of its 8 error words have VKZG_B200_DEVICE_FAILED.
+ * No counterpart in the reference.
+ */
+vkzg_result vkzg_b200_tensor_mul_selftest(const uint32_t *a, const uint32_t *b, uint32_t n, int give_up,
+                                          uint32_t *results, uint32_t *error_words_marked);
+
+/*
  * Sums n_lists lists of m affine points each (points_xy: n_lists * m x 96
  * bytes, list o first; all zero = infinity) with the grid-wide batch-affine
  * tree rounds of the proof path's plan 3.  points_xy NULL: seeded pseudo-random

@@ -46,7 +46,7 @@ EXPORTED_SYMBOLS = (
     "vkzg_b200_server_stats", "vkzg_b200_kernel_launches", "vkzg_b200_digit_table",
     "vkzg_b200_tree_sums_selftest", "vkzg_b200_window_trials", "vkzg_b200_prover_device_bytes",
     "vkzg_b200_grid_sync_selftest",
-    "vkzg_b200_inverse_selftest",
+    "vkzg_b200_inverse_selftest", "vkzg_b200_tensor_mul_selftest",
 )
 NOALLOC_MAX_BLOBS = 16  # VKZG_B200_NOALLOC_MAX_BLOBS
 
@@ -166,6 +166,8 @@ def library():
             L.vkzg_b200_grid_sync_selftest.restype = ctypes.c_int
             L.vkzg_b200_inverse_selftest.argtypes = [ctypes.c_int, ctypes.c_uint32, u32p]
             L.vkzg_b200_inverse_selftest.restype = ctypes.c_int
+            L.vkzg_b200_tensor_mul_selftest.argtypes = [vp, vp, ctypes.c_uint32, ctypes.c_int, vp, u32p]
+            L.vkzg_b200_tensor_mul_selftest.restype = ctypes.c_int
             L.vkzg_b200_kernel_launches.argtypes = []
             L.vkzg_b200_kernel_launches.restype = ctypes.c_uint64
             _lib = L
@@ -461,6 +463,20 @@ def inverse_selftest(n, seed=1):
     out = ctypes.c_uint32()
     _check(library().vkzg_b200_inverse_selftest(int(n), int(seed), ctypes.byref(out)))
     return out.value
+
+
+def tensor_mul_selftest(a, b, give_up=False):
+    """Tensor-core Fp products of operand pairs (n x 12 words each): (5 x n x 12 words,
+    error words marked), see vkzg_b200_tensor_mul_selftest."""
+    import numpy as np
+    a, b = (np.ascontiguousarray(x, dtype=np.uint32) for x in (a, b))
+    if a.ndim != 2 or a.shape[1] != 12 or a.shape != b.shape:
+        raise ValueError("operands: n x 12 words")
+    out = np.zeros((5,) + a.shape, np.uint32)
+    marked = ctypes.c_uint32()
+    _check(library().vkzg_b200_tensor_mul_selftest(_ptr(a), _ptr(b), len(a), int(give_up), _ptr(out),
+                                                   ctypes.byref(marked)))
+    return out, marked.value
 
 
 def kernel_launches():

@@ -5,6 +5,7 @@
 #include "bucket_sum.cuh"
 #include "device_util.cuh"
 #include "kernels.h"
+#include "tensor_mul.cuh"
 
 #include <vector>
 
@@ -514,6 +515,61 @@ extern "C" vkzg_result vkzg_b200_inverse_selftest(int n, uint32_t seed, uint32_t
     cudaFree(d);
     if (rc == VKZG_OK) *mismatched_words = h;
     return rc;
+}
+
+// The tensor-core products (tensor_mul.cuh) of n operand pairs as they are, n a
+// multiple of the block: out[0] = a b and out[1] = a^2 one after another, not
+// reduced below p, then through the pipeline, reduced: out[2] = a b, out[3] = b^2,
+// out[4] = a^2 (n values each).  give_up: then a wait for a product that nothing
+// started, which runs out and marks the error words.
+constexpr int kTmTestThreads = kTmGroup * kTmMaxGroups;
+__global__ void __launch_bounds__(kTmTestThreads) k_tensor_mul_selftest(const Fp *a, const Fp *b, Fp *out, int n,
+                                                                       int give_up, uint32_t *err, uint32_t n_err) {
+    __shared__ __align__(128) uint8_t area[kTmSmem];
+    Tm g = tm_begin(area);
+    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const Fp x = ld_vec(&a[t]), y = ld_vec(&b[t]);
+    st_vec(&out[t], tm_mul<false>(g, x, y));
+    st_vec(&out[n + t], tm_sqr<false>(g, x));
+    tm_push_first(g, x, y);
+    st_vec(&out[2 * (size_t)n + t], tm_push<true>(g, y, y));
+    st_vec(&out[3 * (size_t)n + t], tm_push_sqr<true>(g, x));
+    st_vec(&out[4 * (size_t)n + t], tm_pop<true>(g));
+    if (give_up) tm_pop<false>(g);
+    tm_end(area, err, n_err);
+}
+
+extern "C" vkzg_result vkzg_b200_tensor_mul_selftest(const uint32_t *a, const uint32_t *b, uint32_t n, int give_up,
+                                                     uint32_t *results, uint32_t *error_words_marked) {
+    if (!a || !b || !results || !error_words_marked || n == 0 || n > (1u << 20)) return VKZG_ERR_BADARGS;
+    constexpr uint32_t kErrWords = 8;
+    const size_t blocks = (n + kTmTestThreads - 1) / kTmTestThreads, padded = blocks * kTmTestThreads;
+    Fp *d = nullptr; // a, b, then the five results
+    uint32_t *err = nullptr, h[kErrWords] = {};
+    vkzg_result rc = VKZG_OK;
+    if (cudaMalloc(&d, 7 * padded * sizeof(Fp)) != cudaSuccess || cudaMalloc(&err, sizeof h) != cudaSuccess)
+        rc = VKZG_ERR_MALLOC;
+    if (rc == VKZG_OK && (cudaMemset(d, 0, 2 * padded * sizeof(Fp)) != cudaSuccess ||
+                          cudaMemset(err, 0, sizeof h) != cudaSuccess ||
+                          cudaMemcpy(d, a, n * sizeof(Fp), cudaMemcpyHostToDevice) != cudaSuccess ||
+                          cudaMemcpy(d + padded, b, n * sizeof(Fp), cudaMemcpyHostToDevice) != cudaSuccess))
+        rc = VKZG_ERR_GPU;
+    if (rc == VKZG_OK) {
+        k_tensor_mul_selftest<<<(unsigned)blocks, kTmTestThreads>>>(d, d + padded, d + 2 * padded, (int)padded, give_up,
+                                                                   err, kErrWords);
+        count_launches(1);
+        if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) rc = VKZG_ERR_GPU;
+    }
+    for (size_t k = 0; k < 5 && rc == VKZG_OK; k++)
+        if (cudaMemcpy(results + k * n * 12, d + (2 + k) * padded, n * sizeof(Fp), cudaMemcpyDeviceToHost) != cudaSuccess)
+            rc = VKZG_ERR_GPU;
+    if (rc == VKZG_OK && cudaMemcpy(h, err, sizeof h, cudaMemcpyDeviceToHost) != cudaSuccess) rc = VKZG_ERR_GPU;
+    cudaFree(d);
+    cudaFree(err);
+    if (rc != VKZG_OK) return rc;
+    *error_words_marked = 0;
+    for (uint32_t w : h) *error_words_marked += (w & kSyncFailed) ? 1u : 0u;
+    return VKZG_OK;
 }
 
 // Sums n_lists lists of m points each with the proof path's grid-wide

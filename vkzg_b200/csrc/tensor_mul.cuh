@@ -204,10 +204,12 @@ constexpr int kTmSums = 2 * kTmBytes;
 static_assert(kTmSums + kTmCols <= kTmTmemCols, "the areas fit a group's columns");
 constexpr int kTmMatrixBytes = kTmRowsPad * kTmCols;
 // a block's shared memory: the matrix, then one mbarrier per group (at most
-// kTmMaxGroups), the TMEM address, the flag that a wait gave up, and one count of
-// arrived warps per group
+// kTmMaxGroups) and one for tm_drain, the TMEM address, the flag that a wait gave
+// up, and one count of arrived warps per group
 constexpr int kTmMaxGroups = 2;
-constexpr int kTmCounts = kTmMatrixBytes + 8 * kTmMaxGroups + 8;
+constexpr int kTmDrain = kTmMatrixBytes + 8 * kTmMaxGroups;
+constexpr int kTmWords0 = kTmDrain + 8; // the TMEM address, then the flag
+constexpr int kTmCounts = kTmWords0 + 8;
 constexpr int kTmSmem = kTmCounts + 4 * kTmMaxGroups;
 static_assert(kTmGroup == 128, "a count of four warps per product");
 // polls of a wait for the tensor core (each suspends up to kTmPollNs) before it gives up
@@ -231,9 +233,11 @@ __device__ __forceinline__ Tm tm_begin(uint8_t *area) {
     for (int x = threadIdx.x; x < kTmMatrixBytes / 16; x += blockDim.x)
         reinterpret_cast<uint4 *>(area)[x] = __ldg(&im[x]);
     const uint32_t bars = tm_smem(area) + kTmMatrixBytes;
-    uint32_t *word = reinterpret_cast<uint32_t *>(area + kTmMatrixBytes + 8 * kTmMaxGroups);
-    if (threadIdx.x < kTmMaxGroups)
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars + 8 * threadIdx.x) : "memory");
+    uint32_t *word = reinterpret_cast<uint32_t *>(area + kTmWords0);
+    if (threadIdx.x <= kTmMaxGroups) // tm_drain's takes an arrival from every warp
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bars + 8 * threadIdx.x),
+                     "r"(threadIdx.x < kTmMaxGroups ? 1u : blockDim.x / 32)
+                     : "memory");
     if (threadIdx.x <= kTmMaxGroups) word[1 + threadIdx.x] = 0; // the flag, the counts
     if (threadIdx.x < 32) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tm_smem(word)),
@@ -252,16 +256,41 @@ __device__ __forceinline__ Tm tm_begin(uint8_t *area) {
     return g;
 }
 
+// After a wait gave up (all threads): waits, bounded like every wait, until no
+// product that the block started is in flight any more, so that none reads TMEM or
+// signals an mbarrier that the block no longer owns.  Each warp's first lane, which
+// started that warp's products, commits them to one mbarrier.
+static __device__ __noinline__ void tm_drain(uint32_t bar) {
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0)
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
+                     : "memory");
+    uint32_t ok = 0;
+    for (uint32_t polls = 0; !ok && polls <= kTmPolls; polls++)
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0, %2;\n\t"
+                     "selp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok)
+                     : "r"(bar), "n"(kTmPollNs)
+                     : "memory");
+    __syncwarp();
+}
+
 // End of the block's products (all threads): frees the TMEM; if a wait gave up,
-// marks the launch's error words (err may be null) like a grid barrier does.
+// waits for the products in flight first and marks the launch's error words (err
+// may be null) like a grid barrier does.
 __device__ __forceinline__ void tm_end(uint8_t *area, uint32_t *err, uint32_t n_err) {
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    volatile uint32_t *word = reinterpret_cast<volatile uint32_t *>(area + kTmMatrixBytes + 8 * kTmMaxGroups);
+    volatile uint32_t *word = reinterpret_cast<volatile uint32_t *>(area + kTmWords0);
+    const bool gave_up = word[1] != 0;
+    if (gave_up) {
+        tm_drain(tm_smem(area) + kTmDrain);
+        __syncthreads();
+    }
     if (threadIdx.x < 32)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(word[0]),
                      "n"(kTmMaxGroups * kTmTmemCols));
-    if (word[1] && err)
+    if (gave_up && err)
         for (uint32_t b = threadIdx.x; b < n_err; b += blockDim.x) atomicOr(&err[b], kSyncFailed);
 }
 
@@ -328,7 +357,7 @@ __device__ __forceinline__ void tm_sums(uint32_t t, uint32_t ctl, uint32_t *w) {
                      : "memory");
         if (!ok) { // bounded: after kTmPolls the block's flag is set and no wait of the block polls again
             uint32_t gave_up;
-            const uint32_t flag = sm + kTmMatrixBytes + 8 * kTmMaxGroups + 4;
+            const uint32_t flag = sm + kTmWords0 + 4;
             asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(gave_up) : "r"(flag) : "memory");
             if (gave_up) break;
             if (++polls > kTmPolls) asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(flag), "r"(1u) : "memory");
@@ -403,39 +432,39 @@ __device__ __forceinline__ void tm_put_sqr(const Fp &a, uint32_t t, uint32_t ctl
     sqr_words<6>(z, x.sum);
     tm_put(t + 24, z);
 }
-__device__ __noinline__ Fp tm_mul_call(Fp a, Fp b, uint32_t t, uint32_t ctl) {
+static __device__ __noinline__ Fp tm_mul_call(Fp a, Fp b, uint32_t t, uint32_t ctl) {
     tm_put_mul(a, b, t, ctl);
     tm_start(t, ctl);
     uint32_t w[kTmCols / 2];
     tm_sums(t, ctl, w);
     return tm_result(w);
 }
-__device__ __noinline__ Fp tm_sqr_call(Fp a, uint32_t t, uint32_t ctl) {
+static __device__ __noinline__ Fp tm_sqr_call(Fp a, uint32_t t, uint32_t ctl) {
     tm_put_sqr(a, t, ctl);
     tm_start(t, ctl);
     uint32_t w[kTmCols / 2];
     tm_sums(t, ctl, w);
     return tm_result(w);
 }
-__device__ __noinline__ void tm_push_first_call(Fp a, Fp b, uint32_t t, uint32_t ctl) {
+static __device__ __noinline__ void tm_push_first_call(Fp a, Fp b, uint32_t t, uint32_t ctl) {
     tm_put_mul(a, b, t, ctl);
     tm_start(t, ctl);
 }
-__device__ __noinline__ Fp tm_push_mul_call(Fp a, Fp b, uint32_t t, uint32_t ctl) {
+static __device__ __noinline__ Fp tm_push_mul_call(Fp a, Fp b, uint32_t t, uint32_t ctl) {
     tm_put_mul(a, b, t, ctl);
     uint32_t w[kTmCols / 2];
     tm_sums(t, ctl, w);
     tm_start(t, ctl);
     return tm_result(w);
 }
-__device__ __noinline__ Fp tm_push_sqr_call(Fp a, uint32_t t, uint32_t ctl) {
+static __device__ __noinline__ Fp tm_push_sqr_call(Fp a, uint32_t t, uint32_t ctl) {
     tm_put_sqr(a, t, ctl);
     uint32_t w[kTmCols / 2];
     tm_sums(t, ctl, w);
     tm_start(t, ctl);
     return tm_result(w);
 }
-__device__ __noinline__ Fp tm_pop_call(uint32_t t, uint32_t ctl) {
+static __device__ __noinline__ Fp tm_pop_call(uint32_t t, uint32_t ctl) {
     uint32_t w[kTmCols / 2];
     tm_sums(t, ctl, w);
     return tm_result(w);
