@@ -592,6 +592,7 @@ extern "C" vkzg_result vkzg_b200_tree_sums_selftest(const uint8_t *points_xy, si
     G1A *lists = nullptr, *buf0 = nullptr, *buf1 = nullptr, *sums = nullptr;
     uint32_t *pre = nullptr;
     Fp *others = nullptr, *tot = nullptr, *totinv = nullptr;
+    uint32_t *err = nullptr, h_err = 0;
     vkzg_result rc = VKZG_OK;
     if (cudaMalloc(&lists, total * sizeof(G1A)) != cudaSuccess ||
         cudaMalloc(&buf0, n_lists * (size_t)((m + 1) / 2) * sizeof(G1A)) != cudaSuccess ||
@@ -600,7 +601,8 @@ extern "C" vkzg_result vkzg_b200_tree_sums_selftest(const uint8_t *points_xy, si
         cudaMalloc(&pre, lanes / 32 * slots * 384 * sizeof(uint32_t)) != cudaSuccess ||
         cudaMalloc(&others, lanes * sizeof(Fp)) != cudaSuccess ||
         cudaMalloc(&tot, lanes / 32 * sizeof(Fp)) != cudaSuccess ||
-        cudaMalloc(&totinv, lanes / 32 * sizeof(Fp)) != cudaSuccess) {
+        cudaMalloc(&totinv, lanes / 32 * sizeof(Fp)) != cudaSuccess ||
+        cudaMalloc(&err, sizeof h_err) != cudaSuccess || cudaMemset(err, 0, sizeof h_err) != cudaSuccess) {
         rc = VKZG_ERR_MALLOC;
     }
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -618,10 +620,15 @@ extern "C" vkzg_result vkzg_b200_tree_sums_selftest(const uint8_t *points_xy, si
         cudaEventCreate(&e0);
         cudaEventCreate(&e1);
         cudaEventRecord(e0);
-        launch_tree_sums(lists, (int)n_lists, m, buf0, buf1, pre, others, tot, totinv, slots, blocks, sums, 0);
+        launch_tree_sums(lists, (int)n_lists, m, buf0, buf1, pre, others, tot, totinv, slots, blocks, sums,
+                         err, 0);
         cudaEventRecord(e1);
         if (cudaEventSynchronize(e1) != cudaSuccess || cudaGetLastError() != cudaSuccess) rc = VKZG_ERR_GPU;
     }
+    // a wait of the rounds gave up: their sums are not the lists' sums
+    if (rc == VKZG_OK &&
+        (cudaMemcpy(&h_err, err, sizeof h_err, cudaMemcpyDeviceToHost) != cudaSuccess || (h_err & kSyncFailed)))
+        rc = VKZG_ERR_GPU;
     if (rc == VKZG_OK && ms) {
         float t = 0.f;
         cudaEventElapsedTime(&t, e0, e1);
@@ -645,5 +652,6 @@ extern "C" vkzg_result vkzg_b200_tree_sums_selftest(const uint8_t *points_xy, si
     cudaFree(others);
     cudaFree(tot);
     cudaFree(totinv);
+    cudaFree(err);
     return rc;
 }

@@ -197,7 +197,7 @@ struct FlatSizes {
 };
 FlatSizes flat_sizes(int cap, int windows);
 int launch_tree_sums(const G1A *lists, int n_lists, uint32_t m, G1A *buf0, G1A *buf1, uint32_t *pre, Fp *others,
-                     Fp *tot, Fp *totinv, size_t slots, int blocks, G1A *sums, cudaStream_t s);
+                     Fp *tot, Fp *totinv, size_t slots, int blocks, G1A *sums, uint32_t *err, cudaStream_t s);
 cudaError_t launch_comb_table(const DeviceTables &t, G1A *comb, void *scratch, int windows, cudaStream_t s);
 cudaError_t launch_setup_tables(const uint8_t *d_g1_monomial, G1A *pos, const Fr *roots_fwd, void *scratch,
                                 uint32_t *d_err, cudaStream_t s);

@@ -718,7 +718,7 @@ struct FlatArgs {
     Fp *tot, *totinv;    // per warp: product of all, and its inverse
     size_t slots;
     int n_lists;
-    uint32_t *err; // error words, marked when a wait for the tensor core gives up (may be null)
+    uint32_t *err; // error words, marked when a wait for the tensor core gives up
     uint32_t n_err;
 };
 
@@ -1342,9 +1342,10 @@ const G1A *run_tree_rounds(FlatArgs a, const G1A *first_src, uint32_t *m_io, uin
 
 // Sums of n_lists lists of m points (list o at lists[o m ..]) by the same
 // grid-wide rounds, for tests and profiles of the rounds alone (the lists
-// buffer is not written unless m == 1).  Returns the launches made.
+// buffer is not written unless m == 1).  err: one error word, zeroed by the
+// caller.  Returns the launches made.
 int launch_tree_sums(const G1A *lists, int n_lists, uint32_t m, G1A *buf0, G1A *buf1, uint32_t *pre, Fp *others,
-                     Fp *tot, Fp *totinv, size_t slots, int blocks, G1A *sums, cudaStream_t s) {
+                     Fp *tot, Fp *totinv, size_t slots, int blocks, G1A *sums, uint32_t *err, cudaStream_t s) {
     FlatArgs a;
     memset(&a, 0, sizeof a);
     a.pre = pre;
@@ -1353,6 +1354,8 @@ int launch_tree_sums(const G1A *lists, int n_lists, uint32_t m, G1A *buf0, G1A *
     a.totinv = totinv;
     a.slots = slots;
     a.n_lists = n_lists;
+    a.err = err;
+    a.n_err = 1;
     int launched = 0;
     if (cudaFuncSetAttribute(k_flat_pass2<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStage2Bytes) !=
         cudaSuccess)

@@ -276,8 +276,8 @@ static __device__ __noinline__ void tm_drain(uint32_t bar) {
 }
 
 // End of the block's products (all threads): frees the TMEM; if a wait gave up,
-// waits for the products in flight first and marks the launch's error words (err
-// may be null) like a grid barrier does.
+// waits for the products in flight first and marks the launch's error words like a
+// grid barrier does.
 __device__ __forceinline__ void tm_end(uint8_t *area, uint32_t *err, uint32_t n_err) {
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -290,7 +290,7 @@ __device__ __forceinline__ void tm_end(uint8_t *area, uint32_t *err, uint32_t n_
     if (threadIdx.x < 32)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(word[0]),
                      "n"(kTmMaxGroups * kTmTmemCols));
-    if (gave_up && err)
+    if (gave_up)
         for (uint32_t b = threadIdx.x; b < n_err; b += blockDim.x) atomicOr(&err[b], kSyncFailed);
 }
 
