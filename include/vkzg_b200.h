@@ -48,8 +48,10 @@ const char *vkzg_b200_stage_name(int recovery, int i);
  * d_err (num_blobs words) receives a nonzero word for each blob with a
  * non-canonical element (proofs) or more than 64 missing cells (recovery);
  * those blobs' outputs are unspecified.  Bit 31 of every word of a proof chunk
- * (VKZG_B200_DEVICE_FAILED) means a grid barrier of the chunk's cooperative
- * launches gave up waiting (the host entry points return VKZG_ERR_GPU then).
+ * (VKZG_B200_DEVICE_FAILED) means that a bounded wait of the chunk's kernels gave
+ * up, a wait for the tensor cores or, in the cooperative form, a grid barrier:
+ * the chunk's proofs are unspecified (the host entry points return VKZG_ERR_GPU
+ * then).
  */
 #define VKZG_B200_DEVICE_FAILED 0x80000000u
 vkzg_result vkzg_b200_compute_proofs_device(vkzg_prover *p, uint8_t *d_proofs, const uint8_t *d_blobs,
