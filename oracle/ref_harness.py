@@ -46,10 +46,14 @@ def reference_dir(arg=None):
 
 def build(ref=None, force=False):
     """Compiles both programs; returns their paths, or None when no checkout is
-    given (an empty directory is none)."""
+    given (an empty directory is none).  A checkout without one of the sources
+    raises FileNotFoundError."""
     ref = reference_dir(ref)
-    if not ref or not all(os.path.exists(os.path.join(ref, s)) for _, srcs in PROGRAMS for s in srcs):
+    if not ref or not os.path.isdir(ref) or not os.listdir(ref):
         return None
+    missing = [s for s in [s for _, srcs in PROGRAMS for s in srcs] + HEADERS if not os.path.exists(os.path.join(ref, s))]
+    if missing:
+        raise FileNotFoundError(f"{ref}: no {', '.join(missing)}")
     lib = os.path.join(LIBDIR, "libvkzg.so")
     if not os.path.exists(lib):
         raise FileNotFoundError(f"{lib} is not built (python -m vkzg_b200.build)")
