@@ -243,7 +243,9 @@ vkzg_result vkzg_b200_server_stats(vkzg_server *s, vkzg_server_stats *out, int r
  * warps on each pipe, 15 and 16: Fp multiplies on the FP64 pipe and through one
  * Karatsuba level with four independent chains per thread instead of two
  * (giga-ops/s); 17: as 11, each value inverted by four lanes (the form the
- * proof rounds use), in microseconds.  Best of three timed launches.
+ * proof rounds use), in microseconds; 18 and 19: Fp multiplies reduced on the
+ * tensor cores, one after another and through the pipeline that the proof rounds
+ * use, 20 and 21: Fp squares likewise (giga-ops/s).  Best of three timed launches.
  */
 vkzg_result vkzg_b200_microbench(int which, double *result);
 

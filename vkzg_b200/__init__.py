@@ -492,7 +492,9 @@ def microbench(which):
     16 Fp inversions per SM, variable-time / fixed divstep batches (microseconds);
     12 / 13: Fp multiplies / squares on the FP64 pipe; 14: half the warps on each
     pipe; 15 / 16: FP64-pipe / Karatsuba multiplies with four chains per thread (G/s);
-    17: as 11 with four lanes per inversion (microseconds)."""
+    17: as 11 with four lanes per inversion (microseconds); 18 / 19: Fp multiplies
+    reduced on the tensor cores, one after another / through the pipeline;
+    20 / 21: squares likewise (G/s)."""
     out = ctypes.c_double()
     _check(library().vkzg_b200_microbench(int(which), ctypes.byref(out)))
     return out.value

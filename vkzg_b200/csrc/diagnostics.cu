@@ -186,6 +186,39 @@ __global__ void __launch_bounds__(128) k_probe_fp(uint32_t seed, int iters, uint
     }
 }
 
+// The Fp products reduced on the tensor cores (tensor_mul.cuh), 2 iters per
+// thread on two chains; OP 0: products one after another, 1: products through the
+// pipeline, 2 and 3: squares likewise.
+constexpr int kTmProbeThreads = kTmGroup * kTmMaxGroups;
+template <int OP>
+__global__ void __launch_bounds__(kTmProbeThreads, 2) k_probe_tm(uint32_t seed, int iters, uint32_t *sink, uint32_t *err) {
+    __shared__ __align__(128) uint8_t area[kTmSmem];
+    Tm g = tm_begin(area);
+    Fp a = fp_one(), b = fp_one();
+    a.v[0] ^= seed + threadIdx.x;
+    b.v[1] ^= seed * 3u + blockIdx.x;
+    const Fp c = a;
+    if (OP == 1 || OP == 3) tm_push_first(g, a, c);
+    for (int i = 0; i < iters; i++) {
+        if (OP == 0) {
+            a = tm_mul<false>(g, a, c);
+            b = tm_mul<false>(g, b, c);
+        } else if (OP == 2) {
+            a = tm_sqr<false>(g, a);
+            b = tm_sqr<false>(g, b);
+        } else if (OP == 1) {
+            a = tm_push<false>(g, b, c);
+            b = tm_push<false>(g, a, c);
+        } else {
+            a = tm_push_sqr<false>(g, b);
+            b = tm_push_sqr<false>(g, a);
+        }
+    }
+    if (OP == 1 || OP == 3) a = tm_pop<false>(g);
+    tm_end(area, err, 1);
+    if ((a.v[0] ^ b.v[0]) == 0x12345678u) sink[0] = a.v[1];
+}
+
 // OP 0: fr_mul (CIOS), 1: the Karatsuba product
 template <int OP>
 __global__ void __launch_bounds__(256) k_probe_fr(uint32_t seed, int iters, uint32_t *sink) {
@@ -330,7 +363,7 @@ extern "C" vkzg_result vkzg_b200_bucket_sums_selftest(const uint8_t *points_xy, 
 
 // which: 0 = 32-bit IMAD issue rate (T/s), 1 = Fp multiplies (G/s), 2 = Fr multiplies (G/s)
 extern "C" vkzg_result vkzg_b200_microbench(int which, double *result) {
-    if (!result || which < 0 || which > 17) return VKZG_ERR_BADARGS;
+    if (!result || which < 0 || which > 21) return VKZG_ERR_BADARGS;
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
@@ -338,6 +371,11 @@ extern "C" vkzg_result vkzg_b200_microbench(int which, double *result) {
     uint32_t *sink = nullptr;
     cudaEvent_t e0, e1;
     if (cudaMalloc(&sink, 16) != cudaSuccess) return VKZG_ERR_MALLOC;
+    uint32_t *err = sink + 1, h_err = 0; // the tensor-core products' error word
+    if (cudaMemset(sink, 0, 16) != cudaSuccess) {
+        cudaFree(sink);
+        return VKZG_ERR_GPU;
+    }
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     const int fp_iters = 256, fr_iters = 1024;
@@ -357,6 +395,13 @@ extern "C" vkzg_result vkzg_b200_microbench(int which, double *result) {
             else if (which == 8) k_probe_imad_wide<<<blocks, 256>>>(rep + 1, sink);
             else k_probe_dfma<<<blocks, 256>>>(rep + 1, sink);
             ops = (double)blocks * 256 * 8 * kProbeIters;
+        } else if (which >= 18) {
+            const int blocks = sms * 2;
+            if (which == 18) k_probe_tm<0><<<blocks, kTmProbeThreads>>>(rep + 1, fp_iters, sink, err);
+            else if (which == 19) k_probe_tm<1><<<blocks, kTmProbeThreads>>>(rep + 1, fp_iters, sink, err);
+            else if (which == 20) k_probe_tm<2><<<blocks, kTmProbeThreads>>>(rep + 1, fp_iters, sink, err);
+            else k_probe_tm<3><<<blocks, kTmProbeThreads>>>(rep + 1, fp_iters, sink, err);
+            ops = (double)blocks * kTmProbeThreads * 2 * fp_iters;
         } else if (which != 2 && which != 5) {
             const int blocks = sms * 4;
             if (which == 1) k_probe_fp<0><<<blocks, 128>>>(rep + 1, fp_iters, sink);
@@ -393,7 +438,9 @@ extern "C" vkzg_result vkzg_b200_microbench(int which, double *result) {
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    const bool ok = cudaMemcpy(&h_err, err, sizeof h_err, cudaMemcpyDeviceToHost) == cudaSuccess && !h_err;
     cudaFree(sink);
+    if (!ok) return VKZG_ERR_GPU;
     *result = best;
     return VKZG_OK;
 }
@@ -522,8 +569,7 @@ extern "C" vkzg_result vkzg_b200_inverse_selftest(int n, uint32_t seed, uint32_t
 // reduced below p, then through the pipeline, reduced: out[2] = a b, out[3] = b^2,
 // out[4] = a^2 (n values each).  give_up: then a wait for a product that nothing
 // started, which runs out and marks the error words.
-constexpr int kTmTestThreads = kTmGroup * kTmMaxGroups;
-__global__ void __launch_bounds__(kTmTestThreads) k_tensor_mul_selftest(const Fp *a, const Fp *b, Fp *out, int n,
+__global__ void __launch_bounds__(kTmProbeThreads) k_tensor_mul_selftest(const Fp *a, const Fp *b, Fp *out, int n,
                                                                        int give_up, uint32_t *err, uint32_t n_err) {
     __shared__ __align__(128) uint8_t area[kTmSmem];
     Tm g = tm_begin(area);
@@ -543,7 +589,7 @@ extern "C" vkzg_result vkzg_b200_tensor_mul_selftest(const uint32_t *a, const ui
                                                      uint32_t *results, uint32_t *error_words_marked) {
     if (!a || !b || !results || !error_words_marked || n == 0 || n > (1u << 20)) return VKZG_ERR_BADARGS;
     constexpr uint32_t kErrWords = 8;
-    const size_t blocks = (n + kTmTestThreads - 1) / kTmTestThreads, padded = blocks * kTmTestThreads;
+    const size_t blocks = (n + kTmProbeThreads - 1) / kTmProbeThreads, padded = blocks * kTmProbeThreads;
     Fp *d = nullptr; // a, b, then the five results
     uint32_t *err = nullptr, h[kErrWords] = {};
     vkzg_result rc = VKZG_OK;
@@ -555,7 +601,7 @@ extern "C" vkzg_result vkzg_b200_tensor_mul_selftest(const uint32_t *a, const ui
                           cudaMemcpy(d + padded, b, n * sizeof(Fp), cudaMemcpyHostToDevice) != cudaSuccess))
         rc = VKZG_ERR_GPU;
     if (rc == VKZG_OK) {
-        k_tensor_mul_selftest<<<(unsigned)blocks, kTmTestThreads>>>(d, d + padded, d + 2 * padded, (int)padded, give_up,
+        k_tensor_mul_selftest<<<(unsigned)blocks, kTmProbeThreads>>>(d, d + padded, d + 2 * padded, (int)padded, give_up,
                                                                    err, kErrWords);
         count_launches(1);
         if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) rc = VKZG_ERR_GPU;

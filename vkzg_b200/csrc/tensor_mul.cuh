@@ -18,9 +18,9 @@
 // What bounds it: issue slots.  A fused wide multiply-add holds a scheduler
 // about four cycles and every other instruction one; the word-serial form spends
 // 264 of the former per product, this one 120.  Measured on B200, two blocks of 256
-// threads per SM: products 41.7 to 42.5 G/s one after another and 42.3 (warps
-// counted in) to 45.3 (a barrier per product) in the pipeline below, against 28.7
-// G/s for the scalar form; squares 51 and 52 to 55 against 33.1.  The matrix
+// threads per SM (vkzg_b200_microbench 18 to 21, 4 and 6): products 42.2 G/s one after
+// another and 45.0 in the pipeline below, against 29.2 for the scalar form; squares
+// 48.9 and 53.7 against 33.7.  The matrix
 // product takes 48 cycles of an SM per step of 32 rows.  Tried and slower: the
 // reduction through mma.sync (26.8 G/s), products of 24-bit limbs on the FP64 pipe
 // (25.9) or of 30-bit limbs without carries (29.8) in front of the same reduction.
@@ -308,10 +308,9 @@ __device__ __forceinline__ void tm_put(uint32_t t, const uint32_t *z) {
 // group has put its rows and read the sums of the product before: each warp
 // counts itself in and goes on, and the one that completes the count issues the
 // product.  (A barrier of the group in its place is faster when warps do nothing
-// but push, 806 against 865 cycles a product; in the passes, whose warps drift
-// apart over loads, it cost 1.4 of 9.2 cycles per issued instruction: 20.99 against
-// 20.58 ms for the proofs of 256 blobs.)  Called by whole groups, as is everything
-// below.
+// but push, 47.3 against 44.9 G products/s; in the passes, whose warps drift apart
+// over loads, it is slower: 20.98 against 20.52 ms for the proofs of 256 blobs.)
+// Called by whole groups, as is everything below.
 __device__ __forceinline__ void tm_start(uint32_t t, uint32_t ctl) {
     const uint32_t sm = ctl & ~kTmFlags, grp = threadIdx.x / kTmGroup;
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
