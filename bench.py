@@ -53,37 +53,45 @@ IMAD_FP_MUL_KS, IMAD_FP_SQR_KS = 516, 426
 # the same reduced on the tensor cores, as the grid-wide rounds make them: 108 (63
 # for a square) and 12 word products of two multiply instructions, and one more
 IMAD_FP_MUL_TM, IMAD_FP_SQR_TM = 241, 151
-PHASE_A_TAIL = 10  # lists of at most this many points finish in Jacobian form
 
 
-def phase_a_executed_products_per_output(d):
-    """Fp products and squares plan 3's phase A executes per MSM output with a
+def phase_a_tail(n_blobs, sms):
+    """(points, threads) of the Jacobian tail that ends phase A's tree rounds: lists
+    of at most `points` points are summed by `threads` chains of mixed additions and
+    a tree of additions, longer tails for few blobs (tail_threads and tail_points in
+    vkzg_b200/csrc/proof_kernels.cu)."""
+    lists = 128 * n_blobs
+    return (96, 32) if lists <= 8 * sms else (24, 8) if lists <= 32 * sms else (10, 2)
+
+
+def phase_a_additions_per_output(d, n_blobs, sms):
+    """(affine, mixed, Jacobian) additions of plan 3's phase A per MSM output with a
     digit table of d windows (lists of 64 d points)."""
+    points, threads = phase_a_tail(n_blobs, sms)
     m = 64 * d
     adds = 0
-    while m > PHASE_A_TAIL:
+    while m > points:
         adds += m // 2
         m = (m + 1) // 2
-    madds = max(m - 2, 0)
-    return 6 * adds + 11 * madds + 16
+    return adds, max(m - threads, 0), min(m, threads) - 1
 
 
-def phase_a_executed_imad_per_output(d):
-    """Multiply instructions plan 3's phase A executes per MSM output with d
-    windows: affine additions (5 products + 1 square, reduced on the tensor cores)
-    in tree rounds down to lists of PHASE_A_TAIL points, then mixed additions
-    (7 + 4) on two chains and one Jacobian addition (11 + 5)."""
-    m = 64 * d
-    adds = 0
-    while m > PHASE_A_TAIL:
-        adds += m // 2
-        m = (m + 1) // 2
-    madds = max(m - 2, 0)
-    return (adds * (5 * IMAD_FP_MUL_TM + IMAD_FP_SQR_TM) + (7 * madds + 11) * IMAD_FP_MUL_KS +
-            (4 * madds + 5) * IMAD_FP_SQR_KS)
+def phase_a_executed_products_per_output(d, n_blobs, sms):
+    """Fp products and squares plan 3's phase A executes per MSM output."""
+    adds, madds, jadds = phase_a_additions_per_output(d, n_blobs, sms)
+    return 6 * adds + 11 * madds + 16 * jadds
 
 
-def phase_a_dram_bytes(d, n_blobs):
+def phase_a_executed_imad_per_output(d, n_blobs, sms):
+    """Multiply instructions plan 3's phase A executes per MSM output: affine
+    additions (5 products + 1 square, reduced on the tensor cores), then mixed
+    (7 + 4) and Jacobian additions (11 + 5) of the tail."""
+    adds, madds, jadds = phase_a_additions_per_output(d, n_blobs, sms)
+    return (adds * (5 * IMAD_FP_MUL_TM + IMAD_FP_SQR_TM) + (7 * madds + 11 * jadds) * IMAD_FP_MUL_KS +
+            (4 * madds + 5 * jadds) * IMAD_FP_SQR_KS)
+
+
+def phase_a_dram_bytes(d, n_blobs, sms):
     """DRAM bytes of one plan-3 phase-A pass over n_blobs with a digit table of
     d windows: the per-pair ncu dram__bytes_read + dram__bytes_write of the round
     kernels in a 16-blob, 9-bit-window capture, one kernel per capture
@@ -93,9 +101,10 @@ def phase_a_dram_bytes(d, n_blobs):
     table's exact pair counts, plus the digit recoding and the Jacobian tail
     (0.05 GB per 256 blobs).  For 20 windows at 256 blobs: 30.0 GB."""
     lists = 128 * n_blobs
+    points, _ = phase_a_tail(n_blobs, sms)
     m = 64 * d
     total, first = 0.0, True
-    while m > 10:
+    while m > points:
         pairs = lists * (m // 2)
         per = 893 if first else (546 if lists * m * 96 > 126e6 else 500)
         total += pairs * per
@@ -674,9 +683,10 @@ def run_ours(args, rank, world, local_rank):
     digit = prover.digit_table()
     plan = tuning.get(n, (None,))[0] if n in tuning else None
     executed = products = None
+    sms = prover.gpu_core_count()
     if plan == 3 and digit:
-        executed = 128 * phase_a_executed_imad_per_output(digit[0]) * n / (pa_ms / 1e3) / 1e12
-        products = 128 * phase_a_executed_products_per_output(digit[0]) * n / (pa_ms / 1e3) / 1e9
+        executed = 128 * phase_a_executed_imad_per_output(digit[0], n, sms) * n / (pa_ms / 1e3) / 1e12
+        products = 128 * phase_a_executed_products_per_output(digit[0], n, sms) * n / (pa_ms / 1e3) / 1e9
     stages = dict(stages_acc)
     p_ms = statistics.mean(proof_ms)
     rec_ms = statistics.mean(step_ms) - p_ms
@@ -731,14 +741,14 @@ def run_ours(args, rank, world, local_rank):
                      "algorithmic": "multiply instructions phase A executes: per MSM output 64 D - 1 (D windows) "
                                     "digit-table points summed by affine additions (5 products + 1 square, "
                                     "241 / 151 multiply instructions each, their reduction on the tensor cores) "
-                                    "down to lists of 10, then mixed "
+                                    f"down to lists of {phase_a_tail(n, sms)[0]}, then mixed "
                                     "Jacobian additions",
                      "products_g_per_s": products, "product_rate_alone_g_per_s": product_rate,
                      "scalar_product_rate_g_per_s": scalar_rate,
                      "frac_of_product_rate": products / product_rate if products else None,
                      "reference_algorithm_tera_imad_per_s": reference_work,
                      "work_saved": reference_work / executed if executed else None,
-                     "traffic": phase_a_dram_bytes(digit[0], n) if plan == 3 and digit else None,
+                     "traffic": phase_a_dram_bytes(digit[0], n, sms) if plan == 3 and digit else None,
                      "traffic_unit": "DRAM bytes per phase-A pass over the batch (ncu dram__bytes_read + write "
                                      "per pair from a 16-blob 9-bit-window capture, one kernel each, applied "
                                      "to this table's pair counts)"},
