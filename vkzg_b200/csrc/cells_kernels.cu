@@ -82,7 +82,4 @@ cudaError_t launch_cells(const DeviceTables &t, const uint8_t *blobs, uint8_t *c
     return cudaGetLastError();
 }
 
-cudaError_t configure_cells_kernels() { return cudaSuccess; // at most 32 KB of dynamic shared memory
-}
-
 } // namespace vkzg

@@ -1415,8 +1415,9 @@ __device__ __noinline__ void coop_invert(const Fp *tot, Fp *totinv, uint32_t n, 
 // phase's arguments stay in the kernel's parameters (only the round's lists
 // change from round to round), so the passes compile as in their own kernels.
 template <bool FIRST>
-__device__ __forceinline__ void coop_tree(ScalarMul &t, FlatArgs a, const G1A *first_src, G1A *buf0, G1A *buf1, uint32_t m,
-                                          uint32_t stop, GridSync g) {
+__global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSM) k_coop_tree(FlatArgs a, const G1A *first_src, G1A *buf0,
+                                                               G1A *buf1, uint32_t m, uint32_t stop, GridSync g) {
+    ScalarMul t;
     const uint32_t gl = blockIdx.x * blockDim.x + threadIdx.x, NL = gridDim.x * blockDim.x;
     RoundIO io{first_src, buf0};
     if constexpr (FIRST) {
@@ -1455,12 +1456,6 @@ __device__ __forceinline__ void coop_tree(ScalarMul &t, FlatArgs a, const G1A *f
             if (m > stop && !grid_sync(g)) return;
         }
     }
-}
-template <bool FIRST>
-__global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSM) k_coop_tree(FlatArgs a, const G1A *first_src, G1A *buf0,
-                                                               G1A *buf1, uint32_t m, uint32_t stop, GridSync g) {
-    ScalarMul t;
-    coop_tree<FIRST>(t, a, first_src, buf0, buf1, m, stop, g);
 }
 
 // the buffer holding the lists after run_tree_rounds' rounds from m down to stop
@@ -1978,8 +1973,10 @@ VKZG_COOP_FN void coop_flatb_pass2(ScalarMul &t, FlatBArgs a, RoundIO io, int r,
 // Cooperative form of the shared pair sums and phase B's rounds: one launch,
 // grid barriers between the passes (the arguments stay in the kernel's
 // parameters; only the round's lists change).
-__device__ __forceinline__ void coop_phase_b(ScalarMul &t, DerivArgs da, int has_deriv, FlatBArgs fa, G1A *buf0, G1A *buf1,
-                                             int rounds, GridSync g, uint4 *dyn_smem) {
+__global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSM) k_coop_phase_b(DerivArgs da, int has_deriv, FlatBArgs fa,
+                                                                  G1A *buf0, G1A *buf1, int rounds, GridSync g) {
+    extern __shared__ uint4 dyn_smem[];
+    ScalarMul t;
     const uint32_t gl = blockIdx.x * blockDim.x + threadIdx.x, NL = gridDim.x * blockDim.x;
     if (has_deriv) {
         coop_deriv_pass1(t, da, gl, NL);
@@ -2002,12 +1999,6 @@ __device__ __forceinline__ void coop_phase_b(ScalarMul &t, DerivArgs da, int has
         io.dst = io.dst == buf0 ? buf1 : buf0;
         if (r + 1 < rounds && !grid_sync(g)) return;
     }
-}
-__global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSM) k_coop_phase_b(DerivArgs da, int has_deriv, FlatBArgs fa,
-                                                                  G1A *buf0, G1A *buf1, int rounds, GridSync g) {
-    extern __shared__ uint4 dyn_smem[];
-    ScalarMul t;
-    coop_phase_b(t, da, has_deriv, fa, buf0, buf1, rounds, g, dyn_smem);
 }
 
 int launch_phase_b_coop(const DeviceTables &t, const ProofWork &w, int n, cudaStream_t s) {
@@ -2480,7 +2471,9 @@ VKZG_COOP_FN void coop_flatr_pass2(ScalarMul &t, FlatRArgs a, int r, RedRound &r
 
 // Cooperative form of the reduction's rounds (the Horner step stays its own
 // launch: one output per thread, a different register budget).
-__device__ __forceinline__ void coop_reduce(ScalarMul &t, FlatRArgs a, int rounds, GridSync g, RedRound &rr) {
+__global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSM) k_coop_reduce(FlatRArgs a, int rounds, GridSync g) {
+    __shared__ RedRound rr;
+    ScalarMul t;
     const uint32_t gl = blockIdx.x * blockDim.x + threadIdx.x, NL = gridDim.x * blockDim.x;
     for (int r = 0; r < rounds; r++) {
         coop_flatr_pass1(t, a, r, rr, gl, NL);
@@ -2490,11 +2483,6 @@ __device__ __forceinline__ void coop_reduce(ScalarMul &t, FlatRArgs a, int round
         coop_flatr_pass2(t, a, r, rr, gl, NL);
         if (r + 1 < rounds && !grid_sync(g)) return;
     }
-}
-__global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSM) k_coop_reduce(FlatRArgs a, int rounds, GridSync g) {
-    __shared__ RedRound rr;
-    ScalarMul t;
-    coop_reduce(t, a, rounds, g, rr);
 }
 
 // proofs non-null: the Horner step runs inside stage 9 (k_finish_horner), which
@@ -2630,17 +2618,14 @@ VKZG_COOP_FN void coop_norm_pass1(ScalarMul &t, NormArgs a, uint32_t gl, uint32_
 VKZG_COOP_FN void coop_norm_pass2(ScalarMul &t, NormArgs a, uint32_t gl, uint32_t NL) { norm_pass2_body(t, a, gl, NL); }
 
 // Cooperative form of the ladder's normalisation round.
-__device__ __forceinline__ void coop_norm(ScalarMul &t, NormArgs a, GridSync g) {
+__global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSM) k_coop_norm(NormArgs a, GridSync g) {
+    ScalarMul t;
     const uint32_t gl = blockIdx.x * blockDim.x + threadIdx.x, NL = gridDim.x * blockDim.x;
     coop_norm_pass1(t, a, gl, NL);
     if (!grid_sync(g)) return;
     coop_invert(a.tot, a.totinv, NL >> 5, gl, NL);
     if (!grid_sync(g)) return;
     coop_norm_pass2(t, a, gl, NL);
-}
-__global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSM) k_coop_norm(NormArgs a, GridSync g) {
-    ScalarMul t;
-    coop_norm(t, a, g);
 }
 
 int launch_normalize_flat(const ProofWork &w, int n, cudaStream_t s) {

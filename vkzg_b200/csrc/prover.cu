@@ -33,7 +33,6 @@ using namespace vkzg;
 namespace vkzg {
 cudaError_t configure_proof_kernels();
 cudaError_t configure_recover_kernels();
-cudaError_t configure_cells_kernels();
 int batch_affine_blocks_per_sm();
 size_t reduce_scratch_points(int cap_blobs);
 cudaError_t launch_proofs_timed(const DeviceTables &t, const ProofWork &w, int n, cudaStream_t s,
@@ -708,8 +707,7 @@ vkzg_result vkzg_prover_new(vkzg_prover **out, const vkzg_options *opts) {
     cudaDeviceProp prop;
     if (cudaGetDeviceProperties(&prop, dev) != cudaSuccess) return VKZG_ERR_GPU;
     // Kernel attributes are per device: set them on the device this prover uses.
-    if (configure_proof_kernels() != cudaSuccess || configure_recover_kernels() != cudaSuccess ||
-        configure_cells_kernels() != cudaSuccess)
+    if (configure_proof_kernels() != cudaSuccess || configure_recover_kernels() != cudaSuccess)
         return VKZG_ERR_GPU;
 
     vkzg_prover *p = new (std::nothrow) vkzg_prover();
