@@ -60,3 +60,31 @@ def test_cells_and_recovery_at_the_lines(blobs, oracle):
     for b in (0, 3, 4):
         rc, want = oracle.compute_cells(blobs[b])
         assert rc == 0 and np.array_equal(cells[b], np.asarray(want).reshape(-1)), b
+
+
+def test_device_calls_at_the_lines(blobs, monkeypatch):
+    """The device entry points at the same counts: the bytes of the host calls."""
+    torch = pytest.importorskip("torch")
+    monkeypatch.delenv("VKZG_TABLES_PATH", raising=False)
+    monkeypatch.setenv("VKZG_PLAN", "3")
+    monkeypatch.setenv("VKZG_COMB_BITS", "9")
+    dev = torch.device("cuda", 0)
+    rng = np.random.default_rng(6)
+    present = np.zeros((LARGEST, 128), np.uint8)
+    for b in range(LARGEST):
+        present[b, rng.choice(128, int(rng.integers(64, 128)), replace=False)] = 1
+    with vkzg_b200.Prover(max_batch_size=LARGEST) as p:
+        cells, want = np.zeros((LARGEST, 262144), np.uint8), np.zeros(LARGEST * 6144, np.uint8)
+        assert p.compute_cells_and_proofs_raw(cells, want, blobs, LARGEST) == 0
+        erased = cells.reshape(LARGEST, 128, 2048) * present[:, :, None]
+        d_blobs, d_cells, d_present = (torch.from_numpy(np.ascontiguousarray(a)).to(dev) for a in (blobs, erased, present))
+        stream = torch.cuda.current_stream(dev).cuda_stream
+        for n in COUNTS:
+            d_out, d_ext = (torch.zeros(n * w, dtype=torch.uint8, device=dev) for w in (6144, 262144))
+            d_err, d_miss = (torch.ones(n, dtype=torch.int32, device=dev) for _ in range(2))
+            assert p.compute_proofs_device(d_out.data_ptr(), d_blobs.data_ptr(), d_err.data_ptr(), n, stream) == 0
+            assert p.recover_cells_device(d_ext.data_ptr(), d_cells.data_ptr(), d_present.data_ptr(),
+                                          d_miss.data_ptr(), n, stream) == 0
+            assert not d_err.any() and not d_miss.any(), n
+            assert np.array_equal(d_out.cpu().numpy(), want[:n * 6144]), n
+            assert np.array_equal(d_ext.cpu().numpy(), cells[:n].reshape(-1)), n
