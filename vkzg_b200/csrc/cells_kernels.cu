@@ -22,8 +22,11 @@ namespace vkzg {
 
 // A blob over a cluster of C blocks (cluster_ntt.cuh).  One 512-thread block per
 // blob (128 KB, radix-2 stages) kept a single SM busy: 57 k products, 0.17 ms at
-// the SM's rate, whatever the batch.  Four blocks a blob, or eight while each has
-// an SM of its own.
+// the SM's rate, whatever the batch.  Four blocks a blob, or eight up to SMs / 8
+// blobs (18), the line of recovery (recover_kernels.cu).  Measured, the call on
+// page-locked buffers with eight and with four: 9 blobs 154 and 169 us, 18 blobs
+// 201 and 214, 24 blobs (in parts, which take eight) 229 and 240, 32 blobs 280 and
+// 281, 256 blobs 1528 and 1525.
 constexpr int kCellsThreads = 256;
 
 template <int C>

@@ -33,10 +33,11 @@
 namespace vkzg {
 
 // ---------------------------------------------------------------- stage 1
-// A blob over a cluster of C blocks (cluster_ntt.cuh): four, or eight while each
-// has an SM of its own.  One 512-thread block per blob with radix-2 stages kept
-// one SM busy for 123 us whatever the batch (25 k products are 71 us at an SM's
-// rate), twice that at 256 blobs.
+// A blob over a cluster of C blocks (cluster_ntt.cuh): four, or eight up to SMs / 8
+// blobs (18), the line of recovery.  One 512-thread block per blob with radix-2
+// stages kept one SM busy for 123 us whatever the batch (25 k products are 71 us at
+// an SM's rate), twice that at 256 blobs.  Measured with eight and with four blocks:
+// 18 blobs 39 and 45 us, 24 blobs 40 and 46, 32 blobs 44 and 46, 37 blobs 74 and 62.
 constexpr int kNttThreads = 256;
 
 template <int C>
@@ -236,9 +237,10 @@ __global__ void __launch_bounds__(kReduceThreads) k_reduce(const G1J *__restrict
 // [4 l, 4 l + 4) to S_l and W_l, a suffix scan over the lanes gives
 // T_l = sum of S_m, m >= l, with sum_l l S_l = sum of T_l, l >= 1, and the lanes'
 // W_l + 4 T_l add up in a tree: 20 point operations one after another instead of
-// 57, for 2.3 times the work.  Latency is what counts while every output's warp
-// has a scheduler of its own (n_outputs <= 4 SMs): 0.95 ms a reduction with 8
-// lanes at 1 to 4 blobs.
+// 57, for 2.3 times the work.  Latency is what counts while schedulers are idle.
+// Measured, a reduction with a warp and with 8 lanes per output: 4 blobs (the last
+// count with a scheduler for every warp, n_outputs <= 4 SMs, plan 0's line) 0.29 and
+// 0.95 ms, 5 blobs 0.41 and 0.95, 8 blobs 0.41 and 0.95.
 constexpr int kReduceWarpThreads = 64;
 __device__ __forceinline__ G1J reduce_add(const G1J &a, const G1J &b) { return g1_add(a, b); }
 __device__ __forceinline__ G1J reduce_add(const G1J &a, const G1A &b) { return g1_madd(a, b); }
@@ -310,8 +312,10 @@ __device__ __forceinline__ void butterfly_level(G1J *v, int t, int m) {
 // lanes (and a quarter of a blob's points per block): X^2, Y^2, Y Z, then E^2, B^2,
 // (X + B)^2, then Y3's product: three one after another instead of seven.  Two
 // lanes (half of the points): X^2 and Y^2, Y Z and B^2, E^2 and (X + B)^2, then Y3's:
-// four.  Every block folds the whole blob.  Each while a block has an SM of its
-// own (n <= SMs / LANES); with more blobs the lanes would share schedulers.
+// four.  Every block folds the whole blob.  Each while there are no more blocks than
+// SMs (n <= SMs / LANES).  Measured: 37 blobs 0.46 ms with four lanes and 0.57 with
+// two, 38 blobs 0.67 and 0.57; 74 blobs 0.57 with two and 0.86 with one, 75 blobs 0.82
+// and 0.86, 128 blobs 0.82 and 0.87.
 __device__ __forceinline__ Fp fp_shfl_lane(const Fp &a, int src) {
     Fp r;
 #pragma unroll
@@ -1267,7 +1271,10 @@ __global__ void __launch_bounds__(kFlatThreads, kFlatBlocksPerSM) k_flat_pass2(F
 // a tree over the T.  Two threads and at most 10 points for many lists; while the
 // threads make at most two warps a scheduler, 8 threads and 24 points (32 SMs
 // lists) or a warp and 96 points (8 SMs lists) replace one and three rounds more:
-// 6 blobs 8 rounds and 43 us -> 4 rounds.
+// 6 blobs 8 rounds and 43 us -> 4 rounds.  Measured, phase A with 23 windows: 9 blobs
+// 0.83 ms with a warp and 0.91 with 8 threads, 10 blobs 0.97 and 0.95; 37 blobs 2.13
+// with 8 threads and 2.23 with two, 38 blobs 2.25 and 2.28, 64 blobs 3.38 and 3.39,
+// 75 blobs 3.92 and 3.88.
 constexpr uint32_t kTreeTail = 10, kTreeTail8 = 24, kTreeTail32 = 96;
 static int tail_threads(int lists) {
     const int sms = sm_count();
@@ -2496,7 +2503,8 @@ int launch_reduce_flat(const ProofWork &w, const G1A *buckets, G1J *out, int n_o
         return build_reduce_schedule(h) ? h.n_rounds : 0;
     }();
     // for few outputs the rounds' launches and the Horner chain take longer than
-    // a warp per output (k_reduce_warp), up to two warps a scheduler
+    // a warp per output (k_reduce_warp), up to two warps a scheduler: 9 blobs 0.52
+    // against 0.64 ms (with k_flatr_terms), 10 blobs 0.78 against 0.66
     if (n_out <= 8 * sm_count() && !w.coop) {
         launch_reduce_warp(buckets, proofs ? w.points : out, n_out, s);
         if (!proofs) return 1;
@@ -2528,6 +2536,7 @@ int launch_reduce_flat(const ProofWork &w, const G1A *buckets, G1J *out, int n_o
     }
     // one thread per output is a chain of 317 products: while eight lanes an
     // output make at most two warps a scheduler, the eight-lane form is shorter
+    // (the reduction of 37 blobs 0.88 against 0.93 ms, of 38 blobs 1.01 against 0.95)
     if (proofs && n_out <= 32 * sm_count()) {
         k_flatr_terms<<<n_out * 8 / 64, 64, 0, s>>>(a, w.points);
         k_finish<<<n_out / kCells, kCells, 0, s>>>(w.points, proofs, kPartLevels);

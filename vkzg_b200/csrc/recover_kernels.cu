@@ -27,9 +27,15 @@ namespace vkzg {
 // fused with the pointwise coset shift.  No global scratch is used.  C = 4 (64 KB
 // and a quarter of the per-blob work a block, three blocks on an SM) for
 // throughput: 130 k blobs/s at 256 blobs with one 128 KB block per blob, 143 k in
-// this form.  C = 8 while every block has an SM of its own (n <= SMs / 8): a blob
-// is 0.28 M products, which keep four SMs busy for 0.2 ms, so the call's latency
-// is what eight SMs save.
+// this form.  C = 8 for few blobs: a blob is 0.28 M products, which keep four SMs
+// busy for 0.2 ms, so the call's latency is what eight SMs save.  The line,
+// n <= SMs / 8 (18 blobs), is where the blocks stop being fewer than the SMs; it is
+// below the crossing.  Measured, eight against four blocks a blob, data on the
+// device: 8 blobs 0.229 and 0.340 ms, 15 blobs 0.231 and 0.340 (as many clusters of
+// eight as get SMs to themselves), 16 to 24 blobs 0.254 and 0.342, 32 blobs 0.264 and
+// 0.343, 37 blobs 0.497 and 0.455, 64 blobs 0.537 and 0.499.  A chunk in parts of 8
+// blobs or more on side streams takes eight as well: page-locked, 16 blobs 0.382 and
+// 0.420 ms, 64 blobs 0.735 and 0.840.
 constexpr int kRecQThreads = 256;
 
 // three blocks per SM (80 registers; 64 KB of shared memory each) measured
@@ -167,7 +173,7 @@ static cudaError_t launch_recover_cluster(const DeviceTables &t, const uint8_t *
                                           uint8_t *out, uint32_t *err, int n, cudaStream_t s) {
     static const Fr seven64 = host_seven64();
     static const Fr coset_scale = host_coset_scale();
-    // eight blocks a blob while each has an SM to itself (above)
+    // eight blocks a blob for few blobs (above)
     if (8 * n <= sm_count())
         k_recover_cluster<8><<<8 * n, kRecQThreads, kExtElems / 8 * sizeof(Fr), s>>>(
             cells, present, out, t.roots_fwd, t.roots_inv, t.shift_fwd, t.shift_inv, seven64, coset_scale, err);
