@@ -95,18 +95,18 @@ def phase_a_dram_bytes(d, n_blobs, sms):
     """DRAM bytes of one plan-3 phase-A pass over n_blobs with a digit table of
     d windows: the per-pair ncu dram__bytes_read + dram__bytes_write of the round
     kernels in a 16-blob, 9-bit-window capture, one kernel per capture
-    (profiles/phase_a_dram_traffic_16blobs.md) -- 893 B per pair in round 1,
-    which gathers digit-table points, 546 B in later rounds while a round's
+    (profiles/phase_a_dram_traffic_16blobs.md) -- 884 B per pair in round 1,
+    which gathers digit-table points, 535 B in later rounds while a round's
     input lists exceed the 126 MB L2, 500 B once they fit -- applied to the
     table's exact pair counts, plus the digit recoding and the Jacobian tail
-    (0.05 GB per 256 blobs).  For 20 windows at 256 blobs: 30.0 GB."""
+    (0.05 GB per 256 blobs).  For 19 windows at 256 blobs: 28.1 GB."""
     lists = 128 * n_blobs
     points, _ = phase_a_tail(n_blobs, sms)
     m = 64 * d
     total, first = 0.0, True
     while m > points:
         pairs = lists * (m // 2)
-        per = 893 if first else (546 if lists * m * 96 > 126e6 else 500)
+        per = 884 if first else (535 if lists * m * 96 > 126e6 else 500)
         total += pairs * per
         first = False
         m = (m + 1) // 2
