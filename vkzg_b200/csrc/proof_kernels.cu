@@ -11,7 +11,8 @@
 //                        outputs (k_reduce_warp)            (k_bucket_reduce)
 //   5 k_ladder (fold)    u+- = u[j] +- u[j+64], and for plans 3-4 twice more on
 //                        the cyclic half: the convolution's parts (k_fold_ladder)
-//   6 k_ladder           L[j][d] = 2^(8d) v[j], d < 16      (k_ladder, d < 32: the
+//   6 k_ladder           L[j][d] = 2^(8d) v[j], d < 16, with two or four lanes per
+//                        point for few blobs (k_ladder_lanes; k_ladder, d < 32: the
 //                        taps are split as k1 + k2 z^2 and slots 16..31 read phi(L))
 //   7 k_normalize        Jacobian -> affine, block batch inversion, phi images
 //                                                           (k_normalize)

@@ -808,10 +808,11 @@ void collect_times(const cudaEvent_t *ev, int stages, double *dst) {
 }
 
 // ---------------------------------------------------------------- autotuner
-// Three plans compute identical bytes (section "plan" in launch_proofs_timed):
-// serial Jacobian buckets win for a handful of blobs (more, smaller blocks),
-// batch-affine rounds win once a chunk fills the GPU, and which reduction is
-// faster depends on the chunk size.  The first chunk of each power-of-two size
+// Five plans compute identical bytes (section "plan" in launch_proofs_timed).
+// Plan 3 has measured fastest at every size once its digit table is built; in a
+// prover without the table serial Jacobian buckets win for a handful of blobs
+// (more, smaller blocks) and batch-affine rounds once a chunk fills the GPU, and
+// which reduction is faster depends on the chunk size.  The first chunk of each power-of-two size
 // class is timed under every plan on the stream and the fastest is kept.
 
 constexpr int kPlans = 5;
@@ -885,7 +886,7 @@ cudaError_t run_proofs(vkzg_prover *p, const ProofWork &w, uint32_t n) {
 // max_batch_size reaches it (it builds the table for its larger chunks anyway),
 // at the fewest-window candidate: the window count is chosen at the larger
 // classes.  With the table built, plan 3 measured fastest down to one blob
-// (3.0 against 4.0 ms for plan 0, 3.7 against 6.2 ms at 8 blobs).
+// (1.79 against 1.86 ms for plan 0, 2.41 against 4.94 ms at 8 blobs).
 constexpr uint32_t kCombMinBlobs = 16;
 
 // ------------------------------------------------------------ digit table
@@ -939,9 +940,9 @@ bool ensure_flat_b(vkzg_prover *p) {
     w.flat_slots = z.slots;
     w.flat_blocks = z.blocks;
     // $VKZG_COOP=1: the rounds of each phase as one cooperative launch (10
-    // launches per proof step instead of ~60); measured 3 % slower than the
-    // captured graph of separate launches (the round loop's state pushes the
-    // passes past 128 registers), so it is not the default
+    // launches per proof step instead of ~60); 21.9 against 18.8 ms for the
+    // captured graph of separate launches (256 blobs, 19 windows: the cooperative
+    // kernels make scalar products), so it is not the default
     const char *coop = getenv("VKZG_COOP");
     if (!p->coop_off && coop && atoi(coop) != 0 && coop_supported(z.blocks / (int)p->sm_count) &&
         p->alloc(w.sync, 4))
