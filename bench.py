@@ -504,7 +504,7 @@ def run_ours(args, rank, world, local_rank):
         assert rc == 0 and np.array_equal(want.reshape(-1, EXT), got_cells[pick_r]), "recovery differs from the oracle"
         verified.update({"proofs_vs_oracle": len(pick_p), "recovered_blobs_vs_oracle": len(pick_r)})
 
-    # ---- BASELINE config 1: recovery of 16 blobs keeping exactly 64 of 128 cells,
+    # ---- recovery of 16 blobs keeping exactly 64 of 128 cells,
     # seeded uniform subsets; device-resident and through the C ABI (pinned buffers)
     c1 = None
     if n >= 16:
@@ -661,7 +661,7 @@ def run_ours(args, rank, world, local_rank):
                    "mix": "Poisson arrivals; 1-64 blobs per request (geometric, mean 6); 70% proofs, "
                           "30% recovery with 64-127 cells present"}
         if args.c4_seconds > 0:
-            # BASELINE config 4 as stated: 60 s at the top offered load with the
+            # 60 s at the top offered load with the
             # admission budget at 8 GiB of working set, which binds (3 lanes x 128
             # blobs of proof work in flight would need more)
             top = [max(fractions)]
@@ -788,7 +788,7 @@ def main():
     ap.add_argument("--serve-batch", type=int, default=128, help="the server's max_blobs_per_batch")
     ap.add_argument("--serve-lanes", type=int, default=3, help="the server's lanes")
     ap.add_argument("--c4-seconds", type=float, default=60.0,
-                    help="BASELINE config 4 at the top load with an 8 GiB budget; 0 skips it")
+                    help="the top load under an 8 GiB working-set budget; 0 skips it")
     ap.add_argument("--table-budget-gb", type=float, default=136.0,
                     help="digit-table budget (GiB) unless $VKZG_COMB_BUDGET_GB is set")
     args = ap.parse_args()
